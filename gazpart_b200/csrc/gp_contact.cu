@@ -2,12 +2,15 @@
 // 216-348), compiled without FMA contraction so that every rounded operation matches an
 // IEEE restatement of the reference.
 //
-// One solve is a long chain of dependent FP64 operations (about 16k cycles per function
-// evaluation on a lone lane, 3.0 M evaluations per step at 512^3/16.8 M spheroids), so
-// the phase is bound by how many solves the SMs keep in flight: eight blocks of 128 per
-// SM with the solver's pieces out of line (64 registers) finish the bulk sooner than two
-// blocks with the whole iteration inlined in registers, although each lane then runs
-// its own iteration faster.
+// One solve is a chain of dependent FP64 operations, 1.9 us a step on an idle SM
+// (gp_lm_fast.cuh), and the phase runs as long as its longest solve wherever the pairs
+// fit the lanes: 67 steps of 1,769 solves at 256^3 / 1 M spheroids.  So the solver keeps
+// its problem and state in registers (255, two blocks of 128 per SM, no spills).  At
+// 147,000 solves (512^3 / 16.8 M) four blocks at 128 registers took 0.98 ms against 1.01
+// in the solver alone, and up to 30% longer below 40,000 solves, so two blocks serve all
+// sizes.  Contact phase, before (eight blocks at 64 registers, the state in local memory)
+// and now: 0.26 -> 0.09 ms at 10,000 spheroids, 0.85 -> 0.23 at 1 M, 3.23 -> 1.16 at
+// 16.8 M.
 #include <math_constants.h>
 
 #include "gp_contact.cuh"
@@ -15,9 +18,28 @@
 
 namespace gp {
 
+// Takes up pair e: false when its bodies are proven apart or there is nothing to solve.
+// Out of line, on the caller's copies, so that the solving loop keeps its problem and
+// state in registers; likewise the hand-over records of an earlier pass.
+static __device__ __noinline__ bool take_pair(const InstDev *__restrict__ insts, const PoolView *__restrict__ pv,
+                                              const PairRec *__restrict__ pairs, int64_t e, ContactProb &CP,
+                                              LmState &S) {
+  const PairRec pr = pairs[e];
+  PairBodies B;
+  pair_bodies(insts, *pv, pr.home, pr.near, B);
+  const double vkx = B.c2[0] - B.c1[0], vky = B.c2[1] - B.c1[1], vkz = B.c2[2] - B.c1[2];
+  const Quat &q1 = B.q1, &q2 = B.q2;
+  // symmetry axes (first columns of R(q)); disjoint bodies need no solve
+  const double e1[3] = {1.0 - 2.0 * (q1.c * q1.c + q1.d * q1.d), 2.0 * (q1.b * q1.c + q1.a * q1.d),
+                        2.0 * (q1.b * q1.d - q1.a * q1.c)};
+  const double e2[3] = {1.0 - 2.0 * (q2.c * q2.c + q2.d * q2.d), 2.0 * (q2.b * q2.c + q2.a * q2.d),
+                        2.0 * (q2.b * q2.d - q2.a * q2.c)};
+  if (separated(vkx, vky, vkz, e1, B.a1 * B.a1, B.b1 * B.b1, e2, B.a2 * B.a2, B.b2 * B.b2)) return false;
+  return solve_start(B.a1, B.b1, B.a2, B.b2, B.c1, q1, B.c2, q2, CP, S);
+}
+
 // A solve handed over by an earlier pass: its pair and solver state, and the problem
-// rebuilt from the pool by the same set-up (so to the same values).  Out of line: the
-// solving loop only passes the state it already keeps in local memory.
+// rebuilt from the pool by the same set-up (so to the same values).
 static __device__ __noinline__ void resume_solve(const InstDev *__restrict__ insts, const PoolView *__restrict__ pv,
                                                  const PairRec *__restrict__ pairs, const TailRec *__restrict__ rec,
                                                  int64_t &e, ContactProb &CP, LmState &S) {
@@ -135,23 +157,25 @@ void launch_queue_order(const InstDev *insts, const PoolView *pv, const PairRec 
 
 // collision_interaction.f90:216-348 for every candidate pair: minimum image, contact
 // (ellipsoid_contact_detection), contact-point velocities, NVREL.  Colliding pairs
-// (flag && NVREL < ZERO) are appended.  Persistent warps with lane refill: a lane whose
-// Levenberg-Marquardt solve has returned finishes its pair and takes the next one from
-// a global queue, so warps do not idle on their slowest pair.  order (optional): the
-// first pass takes the pairs in that order (the queue order above); hist (optional):
-// each pair's outcome is recorded there for the next collision phase's order.
+// (flag && NVREL < ZERO) are appended.  Persistent warps with lane refill: lanes whose
+// Levenberg-Marquardt solve has returned finish their pair and take the next one from a
+// global queue.  order (optional): the first pass takes the pairs in that order (the queue
+// order above); hist (optional): each pair's outcome is recorded there for the next
+// collision phase's order.
 //
-// Passes.  A warp runs as long as its slowest lane, and a step at 512^3 with 16.8 M
-// spheroids has about one solve per lane of the persistent grid, so refilling cannot
-// even out solves of 3 to 300 evaluations.  With `out` set, a solve still running after `budget` evaluations is
-// written there (pair and solver state) and the lane takes other work; a further pass
-// of this kernel (`in` set) resumes those solves with every lane busy, under a larger
-// budget or none.  The iterates are the same operations in the same order.
-#ifndef GP_CONTACT_MIN_BLOCKS
-#define GP_CONTACT_MIN_BLOCKS 8
-#endif
+// Finishing and taking a pair cost about as much as a step, with only the lanes that do
+// it active, so a warp waits until eight of its lanes have something to do there, or none
+// has a solve running.  Fewer pairs than lanes are spread over all warps, a few lanes
+// each: lanes of one warp wait for one another at every branch, lanes of different warps
+// do not (64 solves: 0.111 ms in full warps, 0.097 one a warp).
+//
+// Passes.  With `out` set, a solve still running after `budget` evaluations is written
+// there (pair and solver state) and the lane takes other work; a further pass of this
+// kernel (`in` set) resumes those solves under a larger budget or none.  The iterates are
+// the same operations in the same order.
+constexpr int kContactService = 8;
 
-__global__ void __launch_bounds__(128, GP_CONTACT_MIN_BLOCKS) k_contact(const InstDev *__restrict__ insts,
+__global__ void __launch_bounds__(128, 2) k_contact(const InstDev *__restrict__ insts,
                                                     const PoolView *__restrict__ pv,
                                                     const PairRec *__restrict__ pairs,
                                                     const unsigned long long *__restrict__ npairs, int64_t cap_pairs,
@@ -169,69 +193,67 @@ __global__ void __launch_bounds__(128, GP_CONTACT_MIN_BLOCKS) k_contact(const In
                         : (int64_t)min(*npairs, (unsigned long long)cap_pairs);
   const unsigned lane = threadIdx.x & 31u;
   constexpr unsigned kFull = 0xffffffffu;
-  bool active = false, exhausted = false;
-  // With the order, each warp's first batch of 32 is fixed: warp w of block b takes batch
-  // w * gridDim.x + b of the ordered pairs, so that every block holds one warp of the
-  // longest solves, one of the next longest and so on.  Blocks then stay resident until
-  // their longest solves end, as with the unordered queue, instead of short-solve blocks
-  // leaving early and letting the overlapped gather take issue slots from the long
-  // solves.  Later batches come from the counter, after the fixed ones.
-  bool fixed = order != nullptr && in == nullptr;
-  const unsigned long long lanes = (unsigned long long)gridDim.x * blockDim.x;
+  // lanes of a warp that take pairs: as few as cover the pairs with every warp in use
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const unsigned per = (unsigned)min((int64_t)32, max((int64_t)1, (np + warps - 1) / warps));
+  const bool takes = lane < per;
+  bool active = false, done = false, exhausted = false;
+  // Each warp's first batch is fixed: warp w of block b takes batch w * gridDim.x + b of
+  // the ordered pairs, so that every block holds one warp of the longest solves, one of
+  // the next longest and so on.  Later batches come from the counter.
+  bool fixed = true;
   int64_t e = 0;
   ContactProb CP;
   LmState S;
   for (;;) {
-    if (!exhausted) {
-      const unsigned want = __ballot_sync(kFull, !active);
-      if (want) {
+    const unsigned run = __ballot_sync(kFull, active);
+    const unsigned wait = __ballot_sync(kFull, takes && !active && (done || !exhausted));
+    if (run == 0u && wait == 0u) break;
+    if (run == 0u || __popc(wait) >= kContactService) {
+      if (done) {
+        finish_pair(insts, pv, pairs, e, S.x[0], S.x[1], S.nfev, coll, ncoll, cap_coll, cst, ncst, cap_cst, hist,
+                    nhist, st);
+        done = false;
+      }
+      __syncwarp();
+      if (!exhausted) {
+        const unsigned want = __ballot_sync(kFull, takes && !active);
         unsigned long long base = 0;
         if (fixed) {
-          base = ((unsigned long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32ull;
+          base = ((unsigned long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * per;
           fixed = false;
         } else {
           const int leader = __ffs(want) - 1;
           if ((int)lane == leader) base = atomicAdd(queue, (unsigned long long)__popc(want));
-          base = __shfl_sync(kFull, base, leader);
-          if (order != nullptr && in == nullptr) base += lanes;
+          base = __shfl_sync(kFull, base, leader) + (unsigned long long)warps * per;
         }
         if ((int64_t)base >= np) {
           exhausted = true;
-        } else if (!active) {
+        } else if (takes && !active) {
           const int64_t q = (int64_t)base + __popc(want & ((1u << lane) - 1u));
-          if (q < np && in) {
-            resume_solve(insts, pv, pairs, in + q, e, CP, S);
-            active = true;
-          } else if (q < np) {
-            e = order ? (int64_t)order[q] : q;
-            const PairRec pr = pairs[e];
-            PairBodies B;
-            pair_bodies(insts, *pv, pr.home, pr.near, B);
-            const double vkx = B.c2[0] - B.c1[0], vky = B.c2[1] - B.c1[1], vkz = B.c2[2] - B.c1[2];
-            const Quat &q1 = B.q1, &q2 = B.q2;
-            // symmetry axes (first columns of R(q)); disjoint bodies need no solve
-            const double e1[3] = {1.0 - 2.0 * (q1.c * q1.c + q1.d * q1.d), 2.0 * (q1.b * q1.c + q1.a * q1.d),
-                                  2.0 * (q1.b * q1.d - q1.a * q1.c)};
-            const double e2[3] = {1.0 - 2.0 * (q2.c * q2.c + q2.d * q2.d), 2.0 * (q2.b * q2.c + q2.a * q2.d),
-                                  2.0 * (q2.b * q2.d - q2.a * q2.c)};
-            const bool apart =
-                separated(vkx, vky, vkz, e1, B.a1 * B.a1, B.b1 * B.b1, e2, B.a2 * B.a2, B.b2 * B.b2);
-            if (!apart && contact_setup(B.a1, B.b1, B.a2, B.b2, B.c1, q1, B.c2, q2, CP, S.x)) {
-              lm_begin(CP, S);
+          if (q < np) {
+            ContactProb cp;
+            LmState s;
+            if (in) {
+              resume_solve(insts, pv, pairs, in + q, e, cp, s);
               active = true;
+            } else {
+              e = order ? (int64_t)order[q] : q;
+              active = take_pair(insts, pv, pairs, e, cp, s);
+            }
+            if (active) {
+              CP = cp;
+              S = s;
             } else if (hist) {
               record_apart(insts, pv, pairs, e, hist, nhist);
             }
           }
         }
       }
-    }
-    if (!__any_sync(kFull, active)) {
-      if (exhausted) break;
       continue;
     }
     if (!active) continue;
-    if (lm_step(CP, S, kContactTol) == 0) {
+    if (lm_advance(CP, S) == 0) {
       // past the budget the solve moves on to the next pass and the lane takes other
       // work (with the hand-over buffer full, the lane keeps the solve)
       if (out != nullptr && S.nfev >= budget) {
@@ -242,10 +264,10 @@ __global__ void __launch_bounds__(128, GP_CONTACT_MIN_BLOCKS) k_contact(const In
           active = false;
         }
       }
-      continue;
+    } else {
+      active = false;
+      done = true;
     }
-    active = false;
-    finish_pair(insts, pv, pairs, e, S.x[0], S.x[1], S.nfev, coll, ncoll, cap_coll, cst, ncst, cap_cst, hist, nhist, st);
   }
 }
 

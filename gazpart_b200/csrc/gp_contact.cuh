@@ -2,7 +2,7 @@
 // geometry, and what follows a finished contact solve.
 #pragma once
 
-#include "gp_lm.cuh"
+#include "gp_lm_fast.cuh"
 
 namespace gp {
 

@@ -5,7 +5,7 @@
 #include <math_constants.h>
 
 #include "gp_advance.cuh"
-#include "gp_lm.cuh"
+#include "gp_lm_fast.cuh"
 #include "gp_launch.h"
 
 namespace gp {
@@ -221,7 +221,7 @@ __global__ void k_euler_batch(int64_t n, const double *ip, double dt, double *om
   }
 }
 
-__global__ void __launch_bounds__(128, 8) k_contact_batch(int64_t n, const double *shapes, const double *centres, const double *quats,
+__global__ void __launch_bounds__(128, 2) k_contact_batch(int64_t n, const double *shapes, const double *centres, const double *quats,
                                 int32_t *flag, double *e1, double *e2, double *cn) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const double *s = shapes + 4 * i, *c = centres + 6 * i, *q = quats + 8 * i;

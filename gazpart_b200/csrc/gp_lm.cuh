@@ -1,5 +1,6 @@
-// gp_lm.cuh -- ellipsoid contact detection with a register-resident Levenberg-
-// Marquardt solve (FP64), one pair per thread.
+// gp_lm.cuh -- ellipsoid contact detection: the problem, its Levenberg-Marquardt step for
+// any operands (FP64) and the tests around the solve, one pair per thread.  The step that
+// the kernels normally run is lm_step_fast (gp_lm_fast.cuh), with the same operations.
 //
 // ellipsoid_contact_detection.f90:1-187 parametrises the common normal by two angles
 // and minimises the squared components of the gap between the two support points
@@ -17,34 +18,15 @@
 
 namespace gp {
 
-// Linkage of the solver's building blocks.  Out-of-line calls keep the register count
-// of the pair-search and batch kernels low; GP_LM_INLINE folds the whole solve into
-// its caller, which shortens the dependent-latency chain of one iteration.
-#ifdef GP_LM_INLINE
-#define GP_LM_FN static __device__ __forceinline__
-#else
+// The general step is out of line (its callers, gp_lm_fast.cuh, reach it on rare operands
+// only), and so is what runs once per solve; the pieces of one step are folded into it.
 #define GP_LM_FN static __device__ __noinline__
-#endif
-// The pieces of one iteration are folded into the iteration itself.
 #define GP_LM_INNER static __device__ __forceinline__
-// Once per solve (set-up and the final contact test): out of line in every build, so
-// that they do not add to the register pressure of the iteration they bracket.
 #define GP_LM_COLD static __device__ __noinline__
 
-// Correctly rounded FP64 division and square root of the solver, one place for every
-// site of the iteration.  They are in line by default.  Out of line
-// (GP_LM_CALLED_ARITH) each site becomes a call and the iteration's code shrinks by a
-// quarter, but on the B200 the bulk of 150k solves like those of the 512^3 /
-// 16.8 M-spheroid workload then took 4.45 ms against 3.72 ms in line: the calls cost
-// more than the smaller code saves once the norm's rare paths are out of line
-// (lm_enorm).
-#ifdef GP_LM_CALLED_ARITH
-#define GP_LM_ARITH static __device__ __noinline__
-#else
-#define GP_LM_ARITH static __device__ __forceinline__
-#endif
-GP_LM_ARITH double lm_div(double a, double b) { return a / b; }
-GP_LM_ARITH double lm_sqrt(double a) { return sqrt(a); }
+// Correctly rounded FP64 division and square root of the solver.
+GP_LM_INNER double lm_div(double a, double b) { return a / b; }
+GP_LM_INNER double lm_sqrt(double a) { return sqrt(a); }
 
 // MINPACK's scaled Euclidean norm (minpack_reduc.f90:180-232): three accumulators
 // for tiny, mid-range and huge components.
@@ -141,12 +123,7 @@ CT_QUAL double ct_poly_cos(double z) {
  * k*P1 and k*P2 are exact for |k| < 2^20; the three parts are fdlibm's published
  * pio2_1, pio2_2 and pio2_2t, e_rem_pio2.c), Taylor polynomials (coefficients 1/n!) on
  * [-pi/4, pi/4]. */
-#ifdef GP_LM_INLINE
-#define CT_SINCOS_QUAL CT_QUAL
-#else
-#define CT_SINCOS_QUAL inline __host__ __device__ __noinline__
-#endif
-CT_SINCOS_QUAL void ct_sincos(double x, double *s, double *c) {
+inline __host__ __device__ __noinline__ void ct_sincos(double x, double *s, double *c) {
   if (!(fabs(x) < 1.0e9)) {
     *s = x - x + (0.0 / 0.0 + x * 0.0);
     *c = *s;
@@ -225,23 +202,6 @@ struct ContactProb {
   // entry k of body W's matrix, coordinate i of body W's centre
   template <int W> __device__ __forceinline__ double e(int k) const { return W == 0 ? e1[k] : e2[k]; }
   template <int W> __device__ __forceinline__ double b(int i) const { return W == 0 ? b1[i] : b2[i]; }
-};
-
-// The same problem held in shared memory, one column per lane of a 128-thread block
-// (entry m of the lane's problem at base[m * kProbLanes]; m = 0..8 E1, 9..17 E2,
-// 18..20 b1, 21..23 b2): the solve reads it there and keeps its registers for its state.
-constexpr int kProbLanes = 128;
-constexpr int kProbWords = 24;
-struct SmemProb {
-  double* base;
-  template <int W> __device__ __forceinline__ double e(int k) const { return base[(W * 9 + k) * kProbLanes]; }
-  template <int W> __device__ __forceinline__ double b(int i) const { return base[(18 + W * 3 + i) * kProbLanes]; }
-  __device__ __forceinline__ void store(const ContactProb& P) const {
-#pragma unroll
-    for (int k = 0; k < 9; ++k) { base[k * kProbLanes] = P.e1[k]; base[(9 + k) * kProbLanes] = P.e2[k]; }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) { base[(18 + i) * kProbLanes] = P.b1[i]; base[(21 + i) * kProbLanes] = P.b2[i]; }
-  }
 };
 
 // Everything the residual at x computes that the Jacobian at the same x needs again:
@@ -809,22 +769,5 @@ GP_LM_COLD bool contact_finish(double a1, double bb1, double a2, double bb2, con
 }
 
 constexpr double kContactTol = 1.4901161193847656e-08;   // sqrt(epsilon(1.0_8))
-
-// ellipsoid_contact_detection.f90:1-187 for one pair, start to finish.
-GP_LM_FN bool contact_detection(double a1, double bb1, double a2, double bb2,
-                                                      const double c1[3], const Quat& q1, const double c2[3],
-                                                      const Quat& q2, double ept1[3], double ept2[3], double cn[3]) {
-  ContactProb P;
-  LmState S;
-  if (!contact_setup(a1, bb1, a2, bb2, c1, q1, c2, q2, P, S.x)) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) { ept1[i] = CUDART_NAN; ept2[i] = CUDART_NAN; cn[i] = CUDART_NAN; }
-    return false;
-  }
-  lm_begin(P, S);
-  while (lm_step(P, S, kContactTol) == 0) {
-  }
-  return contact_finish(a1, bb1, a2, bb2, q1, q2, P, S.x, ept1, ept2, cn);
-}
 
 }  // namespace gp

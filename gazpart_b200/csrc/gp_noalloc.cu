@@ -36,7 +36,7 @@
 #include <mutex>
 
 #include "../../include/gazpart_gpu.h"
-#include "gp_lm.cuh"
+#include "gp_lm_fast.cuh"
 
 namespace gp {
 namespace {
@@ -76,7 +76,7 @@ __host__ __device__ Regions regions(double *base) {
 // ellipsoid_contact_detection.f90:1-187 for n pairs held in the staging array.  Shapes
 // arrive as (emaj1, apr1, emaj2, apr2); the minor semi-axis emaj/apr is formed here with
 // the same correctly rounded division the context-based entry point does on the host.
-__global__ void __launch_bounds__(128, 4) k_contact_batch_staged(int64_t n, double *base) {
+__global__ void __launch_bounds__(128, 2) k_contact_batch_staged(int64_t n, double *base) {
   const Regions r = regions(base);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const double *s = r.shapes + 4 * i, *c = r.centres + 6 * i, *q = r.quats + 8 * i;
