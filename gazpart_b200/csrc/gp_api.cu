@@ -31,6 +31,7 @@ using namespace gp;
     if (e_ != cudaSuccess) {                                                                      \
       std::fprintf(stderr, "gazpart_b200: %s failed: %s (%s:%d)\n", #call, cudaGetErrorString(e_), \
                    __FILE__, __LINE__);                                                           \
+      cudaGetLastError();   /* reported here, not again by a later launch check */                  \
       return e_ == cudaErrorMemoryAllocation ? GP_ENOMEM : GP_ECUDA;                              \
     }                                                                                             \
   } while (0)
@@ -212,6 +213,36 @@ int ensure_scratch(gp_ctx *c, size_t count) {
   GP_TRY(dalloc(&c->d_scratch, count));
   c->scratch_count = count;
   return GP_OK;
+}
+
+// The 13 state columns back to back, n values each.
+StateCols cols_at(double *base, int64_t n) {
+  StateCols k;
+  for (int i = 0; i < kNState; ++i) k.p[i] = base + (size_t)i * n;
+  return k;
+}
+
+// The caller's device columns, where the copy kernels may access them directly: memory of
+// this device, aligned.  False otherwise (then cudaMemcpy moves them, or reports why not).
+bool direct_cols(const gp_ctx *c, const double *const *cols, StateCols *out) {
+  for (int i = 0; i < kNState; ++i) {
+    cudaPointerAttributes a;
+    if (!cols[i] || ((uintptr_t)cols[i] & 7u) || cudaPointerGetAttributes(&a, cols[i]) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (a.type != cudaMemoryTypeDevice || a.device != c->device) return false;
+    out->p[i] = const_cast<double *>(cols[i]);
+  }
+  return true;
+}
+
+void read_state(gp_ctx *c, const StateCols &out, int64_t count, unsigned mask = kAllStateCols, int only = -1) {
+  launch_read_state(c->d_inst, c->d_pv, c->d_pv_alt, c->cap, c->n_slots, only, out, count, c->stream, mask);
+}
+
+void write_state(gp_ctx *c, const StateCols &in, int64_t count, unsigned mask = kAllStateCols) {
+  launch_write_state(c->d_inst, c->d_pv, c->d_pv_alt, c->cap, c->n_slots, in, count, c->stream, mask);
 }
 
 void drop_graph(gp_ctx *c) {
@@ -1138,9 +1169,16 @@ int gp_add_class(gp_ctx *c, int32_t field, int64_t n, const double *const *cols,
 int gp_download_class(gp_ctx *c, int32_t ig, double *const *cols, int32_t on_device) {
   if (!c || !cols || ig < 1 || ig > (int)c->live.size() || !c->live[ig - 1]) return GP_EBADARG;
   const int64_t n = c->insts[ig - 1].count;
+  StateCols direct;
+  if (on_device && direct_cols(c, cols, &direct)) {
+    read_state(c, direct, n, kAllStateCols, ig - 1);
+    GP_CK(cudaGetLastError());
+    GP_CK(cudaStreamSynchronize(c->stream));
+    return GP_OK;
+  }
   GP_TRY(ensure_scratch(c, (size_t)kNState * n));
   double *tmp = c->d_scratch;
-  launch_gather_state(c->d_inst, c->d_pv, c->n_slots, ig - 1, tmp, c->d_fluid_cols, nullptr, n, c->stream);
+  read_state(c, cols_at(tmp, n), n, kAllStateCols, ig - 1);
   GP_CK(cudaGetLastError());
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   for (int k = 0; k < kNState; ++k)
@@ -1319,12 +1357,19 @@ int gp_download_state(gp_ctx *c, int64_t n, double *const *cols, double *const *
   if (fluid && !c->prm.store_fluid) return GP_EBADARG;
   // the context's scratch buffer, kept between calls: a fresh allocation and its
   // release (which waits for the device) would cost more than the gather itself
+  StateCols direct;
+  if (on_device && !fluid && direct_cols(c, cols, &direct)) {
+    read_state(c, direct, n);
+    GP_CK(cudaGetLastError());
+    GP_CK(cudaStreamSynchronize(c->stream));
+    return GP_OK;
+  }
   const size_t per = (size_t)kNState + (fluid ? kNFluid : 0);
   GP_TRY(ensure_scratch(c, per * n));
   double *tmp = c->d_scratch;
-  launch_gather_state(c->d_inst, c->d_pv, c->n_slots, -1, tmp, c->d_fluid_cols,
-                      fluid ? tmp + (size_t)kNState * n : nullptr, n,
-                      c->stream);
+  read_state(c, cols_at(tmp, n), n);
+  if (fluid)
+    launch_fluid_out(c->d_inst, c->d_pv, c->n_slots, c->d_fluid_cols, tmp + (size_t)kNState * n, n, c->stream);
   GP_CK(cudaGetLastError());
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   for (int k = 0; k < kNState; ++k)
@@ -1338,9 +1383,13 @@ int gp_download_state(gp_ctx *c, int64_t n, double *const *cols, double *const *
 
 int gp_put_state(gp_ctx *c, int64_t n, const double *const *cols, int32_t on_device) {
   if (!c || !cols || n != c->n) return GP_EBADARG;
-  GP_TRY(ensure_scratch(c, (size_t)kNState * n));
-  for (int k = 0; k < kNState; ++k) GP_TRY(copy_in(c, c->d_scratch + (size_t)k * n, cols[k], n, on_device));
-  launch_scatter_state(c->d_inst, c->d_pv, c->n_slots, c->d_scratch, n, c->stream);
+  StateCols in;
+  if (!on_device || !direct_cols(c, cols, &in)) {
+    GP_TRY(ensure_scratch(c, (size_t)kNState * n));
+    for (int k = 0; k < kNState; ++k) GP_TRY(copy_in(c, c->d_scratch + (size_t)k * n, cols[k], n, on_device));
+    in = cols_at(c->d_scratch, n);
+  }
+  write_state(c, in, n);
   GP_CK(cudaGetLastError());
   GP_CK(cudaStreamSynchronize(c->stream));
   c->fluid_ok = false;
@@ -1374,20 +1423,18 @@ int gp_step_host(gp_ctx *c, int64_t n, const double *const *in_cols, double *con
   }
   GP_CK(cudaEventRecord(ev[2], c->side));                 // every column is in
   GP_CK(cudaStreamWaitEvent(c->stream, ev[1], 0));
-  launch_scatter_state(c->d_inst, c->d_pv, c->n_slots, tmp, n, c->stream, kColsPos);
+  write_state(c, cols_at(tmp, n), n, kColsPos);
   GP_CK(cudaGetLastError());
   GP_TRY(enqueue_gather(c, c->stream));
   GP_CK(cudaStreamWaitEvent(c->stream, ev[2], 0));
-  launch_scatter_state(c->d_inst, c->d_pv, c->n_slots, tmp, n, c->stream, kAllStateCols & ~kColsPos);
+  write_state(c, cols_at(tmp, n), n, kAllStateCols & ~kColsPos);
   GP_CK(cudaGetLastError());
   GP_TRY(enqueue_integrate(c));
-  launch_gather_state(c->d_inst, c->d_pv, c->n_slots, -1, tmp, c->d_fluid_cols, nullptr, n, c->stream,
-                      kColsPosQuat);
+  read_state(c, cols_at(tmp, n), n, kColsPosQuat);
   GP_CK(cudaGetLastError());
   GP_CK(cudaEventRecord(ev[3], c->stream));
   GP_TRY(enqueue_collision(c));
-  launch_gather_state(c->d_inst, c->d_pv, c->n_slots, -1, tmp, c->d_fluid_cols, nullptr, n, c->stream,
-                      kColsVelSpin);
+  read_state(c, cols_at(tmp, n), n, kColsVelSpin);
   GP_CK(cudaGetLastError());
   GP_CK(cudaEventRecord(ev[4], c->stream));
   GP_CK(cudaStreamWaitEvent(c->side, ev[3], 0));
@@ -1406,8 +1453,7 @@ int gp_step_host(gp_ctx *c, int64_t n, const double *const *in_cols, double *con
   GP_TRY(read_status(c, &h));
   GP_TRY(resume_after_halt(c, h, &halted));
   if (halted) {
-    launch_gather_state(c->d_inst, c->d_pv, c->n_slots, -1, tmp, c->d_fluid_cols, nullptr, n, c->stream,
-                        kColsVelSpin);
+    read_state(c, cols_at(tmp, n), n, kColsVelSpin);
     GP_CK(cudaGetLastError());
     for (int k = 0; k < kNState; ++k)
       if ((kColsVelSpin >> k) & 1u)
@@ -2000,7 +2046,7 @@ int gp_autotune(gp_ctx *c, int32_t *grids_out) {
   GP_TRY(dalloc(&save, (size_t)kNState * n));
   const bool colstats = c->colstats;   // the trials add nothing to the statistics
   c->colstats = false;
-  launch_gather_state(c->d_inst, c->d_pv, c->n_slots, -1, save, c->d_fluid_cols, nullptr, n, c->stream);
+  read_state(c, cols_at(save, n), n);
   GP_CK(cudaGetLastError());
   static const int kMult[] = {1, 2, 4, 8, 16};
   static const int kPhase[GP_NTUNE] = {GP_PHASE_GATHER, GP_PHASE_INTEGRATE, GP_PHASE_BIN, GP_PHASE_SEARCH};
@@ -2072,7 +2118,7 @@ int gp_autotune(gp_ctx *c, int32_t *grids_out) {
   }
   drop_graph(c);
   if (!rc) {
-    launch_scatter_state(c->d_inst, c->d_pv, c->n_slots, save, n, c->stream);
+    write_state(c, cols_at(save, n), n);
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(c->stream) != cudaSuccess) rc = GP_ECUDA;
   }
   cudaFree(save);

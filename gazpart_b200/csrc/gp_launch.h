@@ -103,19 +103,31 @@ void launch_match(const CollRec *coll, const unsigned long long *ncoll, int64_t 
                   unsigned long long *best2, int8_t *matched, int8_t *state, Status *st, cudaStream_t s);
 void launch_field_layout(void *dst, int prec, int nx, int ny, int nz, int ncomp, int comp, const double *src,
                          int src_layout, int ghost_mode, cudaStream_t s);
-// state columns as bits (x y z u v w qa qb qc qd ox oy oz = bits 0..12)
+void launch_retire(const PoolView *pv, int64_t n, int inst, cudaStream_t s);
+void launch_init_pool(const PoolView *pv, int64_t begin, int64_t n, int inst, const double *cols,
+                      const double *pcs, int64_t ld, int64_t src, cudaStream_t s);
+void launch_connectivity(int nxb, int nyb, int nzb, int periodicity, int32_t *ncon, int32_t *con, cudaStream_t s);
+
+// --- gp_state.cu: the state columns between the caller's order and the pool's ---
+// state columns as bits (x y z u v w qa qb qc qd ox oy oz = bits 0..12); the copies take
+// these five sets
 constexpr unsigned kAllStateCols = (1u << kNState) - 1u;
 constexpr unsigned kColsPosQuat = 0x3C7u;    // x y z qa qb qc qd: final once the integrate is done
 constexpr unsigned kColsVelSpin = 0x1C38u;   // u v w ox oy oz: the response may still change them
 constexpr unsigned kColsPos = 0x7u;          // x y z: all the gather reads
-void launch_gather_state(const InstDev *insts, const PoolView *pv, int64_t n, int only, double *out,
-                         double *const *fluid_cols, double *fluid_out, int64_t count, cudaStream_t s,
-                         unsigned cols = kAllStateCols);
-void launch_retire(const PoolView *pv, int64_t n, int inst, cudaStream_t s);
-void launch_scatter_state(const InstDev *insts, const PoolView *pv, int64_t n, const double *cols,
-                          int64_t count, cudaStream_t s, unsigned mask = kAllStateCols);
-void launch_init_pool(const PoolView *pv, int64_t begin, int64_t n, int inst, const double *cols,
-                      const double *pcs, int64_t ld, int64_t src, cudaStream_t s);
-void launch_connectivity(int nxb, int nyb, int nzb, int periodicity, int32_t *ncon, int32_t *con, cudaStream_t s);
+// (kAllStateCols & ~kColsPos is the fifth)
+struct StateCols {
+  double *p[kNState];   // device pointers; the entries outside the copy's set are not used
+};
+// alt: the pool's other buffer, of capacity cap, used as workspace (its contents are dead
+// between two advances); count: the caller's entries per column; only >= 0: that class
+// alone, at offset 0.
+void launch_read_state(const InstDev *insts, const PoolView *pv, const PoolView *alt, int64_t cap, int64_t n,
+                       int only, const StateCols &out, int64_t count, cudaStream_t s,
+                       unsigned mask = kAllStateCols);
+void launch_write_state(const InstDev *insts, const PoolView *pv, const PoolView *alt, int64_t cap, int64_t n,
+                        const StateCols &in, int64_t count, cudaStream_t s, unsigned mask = kAllStateCols);
+void launch_fluid_out(const InstDev *insts, const PoolView *pv, int64_t n, double *const *fluid, double *fout,
+                      int64_t count, cudaStream_t s);
 
 }  // namespace gp
