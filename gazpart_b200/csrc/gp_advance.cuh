@@ -617,13 +617,13 @@ __device__ __forceinline__ float pick4(const float f[4], int k) {
 // (Kahan) sum of the 64 products.  mode: 0 no gather, 1 cooperative (contiguous row),
 // 2 left to the lane itself.
 __device__ __forceinline__ void gather_warp_fp32(const InstDev* __restrict__ insts, int mode, int inst,
-                                                 int64_t b, float al, float be, float ga, int64_t j0,
+                                                 int64_t b, float al, float be, float ga, int64_t j0, int run,
                                                  double* const* __restrict__ fluid) {
   constexpr unsigned kFull = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int t = lane & 7, k = t >> 1, half = t & 1;
 #pragma unroll 1
-  for (int g = 0; g < 8; ++g) {
+  for (int g = 0; 4 * g < run; ++g) {
     const int o = g * 4 + (lane >> 3);
     const int mo = __shfl_sync(kFull, mode, o);
     const int io = __shfl_sync(kFull, inst, o);
@@ -680,14 +680,90 @@ __device__ __forceinline__ void gather_warp_fp32(const InstDev* __restrict__ ins
   }
 }
 
+// Warp-cooperative FP64 gather for the 32 particles of one warp, in the reference's order
+// of operations (interp_lag3.f90:196-288).  Sixteen lanes serve one particle: lane t takes
+// z plane t >> 2 and the component pair t & 3 (three pairs; the fourth lane of each four
+// idles), so that one load instruction fetches 48 contiguous bytes of eight points where a
+// lane on its own touched 32 scattered sectors, and a lane has its 16 loads in flight at
+// once.  Each lane sums its plane, x then y; the planes are then added in order across the
+// lanes.  The 12 weights are formed one per lane and shared.  buf: 6 x 32 results, written
+// out column by column.
+// What bounds it then is one L1 line per stencil point (64 a particle) at the L1's rate of
+// about one a cycle.  Measured (B200, 256^3 field, 1 M particles, one-step graphs): 0.61 ms
+// by single lanes -> 0.39; three or four blocks per SM (80, 64 registers) 0.46 and 0.42.
+__device__ __forceinline__ void gather_warp_fp64(const InstDev* __restrict__ insts, int mode, int inst, int64_t b,
+                                                 double al, double be, double ga, int64_t j0, int run,
+                                                 double* buf, double* const* __restrict__ fluid) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31, base = lane & 16;
+  const int kk = (lane >> 2) & 3, c = lane & 3;
+  // lane t forms weight t & 3 of axis t >> 2 (lag3_w's factors, in its order)
+  const double w0 = c == 0 ? -1. / 6. : (c == 1 ? 1. / 2. : (c == 2 ? -1. / 2. : 1. / 6.));
+#pragma unroll 1
+  for (int g = 0; 2 * g < run; ++g) {
+    const int o = 2 * g + (lane >> 4);
+    const int mo = __shfl_sync(kFull, mode, o);
+    if (!__any_sync(kFull, mo == 1)) continue;
+    const int io = __shfl_sync(kFull, inst, o);
+    const long long bo = __shfl_sync(kFull, (long long)b, o);
+    const double ax = __shfl_sync(kFull, al, o), ay = __shfl_sync(kFull, be, o), az = __shfl_sync(kFull, ga, o);
+    const double a = kk == 0 ? ax : (kk == 1 ? ay : az);
+    const double w = w0 * (a - (c == 3 ? 1. : 2.)) * (c < 2 ? a - 1. : a) * (c == 0 ? a : a + 1.);
+    double fx[4], fy[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      fx[i] = __shfl_sync(kFull, w, base + i);
+      fy[i] = __shfl_sync(kFull, w, base + 4 + i);
+    }
+    const double fz = __shfl_sync(kFull, w, base + 8 + kk);
+    double y0 = 0.0, y1 = 0.0;
+    if (mo == 1 && c < 3) {
+      const InstDev& I = insts[io];
+      const int64_t sy = I.nx + 3, sz = (int64_t)(I.ny + 4) * sy;
+      const double2* __restrict__ p =
+          reinterpret_cast<const double2*>(static_cast<const double*>(I.field) + (bo + kk * sz) * kFieldStride) + c;
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        double2 v[4];
+#pragma unroll
+        for (int ii = 0; ii < 4; ++ii) v[ii] = __ldg(p + (jj * sy + ii) * (kFieldStride / 2));
+        const double x0 = fx[0] * v[0].x + fx[1] * v[1].x + fx[2] * v[2].x + fx[3] * v[3].x;
+        const double x1 = fx[0] * v[0].y + fx[1] * v[1].y + fx[2] * v[2].y + fx[3] * v[3].y;
+        y0 = (jj == 0) ? fy[0] * x0 : y0 + fy[jj] * x0;
+        y1 = (jj == 0) ? fy[0] * x1 : y1 + fy[jj] * x1;
+      }
+      y0 = fz * y0;
+      y1 = fz * y1;
+    }
+    double z0 = y0, z1 = y1;
+#pragma unroll
+    for (int d = 4; d <= 12; d += 4) {
+      z0 = z0 + __shfl_down_sync(kFull, y0, d);
+      z1 = z1 + __shfl_down_sync(kFull, y1, d);
+    }
+    if (kk == 0 && c < 3) {
+      buf[(2 * c) * 32 + o] = z0;
+      buf[(2 * c + 1) * 32 + o] = z1;
+    }
+  }
+  __syncwarp();
+  if (mode == 1) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) fluid[k][j0 + lane] = buf[k * 32 + lane];
+  }
+  __syncwarp();
+}
+
 // ADV_PARTICLE_ELLP, first half: the six field components at x_n
 // (adv_particle_new.f90:139-206) of the particle that the next integrate pass will
 // place in slot j, perm[j] of the current buffer (the last binning's cell order, so
 // that neighbouring stencils are gathered together).  Reads only positions, instance
 // and id, so it may run while the collision phase updates velocities.  kMixed: every
-// instance holds an FP32 field (warp-cooperative gather); otherwise FP64 fields,
-// gathered per lane in the reference's summation order.
-// Each warp takes the next 32 slots from *ticket (zero at launch), so the slots in
+// instance holds an FP32 field; otherwise FP64 fields, in the reference's summation order.
+// Both gathers are warp-cooperative; stencils mirrored at a wall (not contiguous in x) are
+// left to their own lane.
+// Each warp takes the next `run` slots (a multiple of 4, at most 32; gather_run) from
+// *ticket (zero at launch), so the slots in
 // flight at any time are one contiguous run of the cell order whatever the grid: the
 // field rows that neighbouring stencils share stay in L2 between their uses, where a
 // grid-stride loop over many blocks spreads the resident warps over the pool.
@@ -695,23 +771,34 @@ __device__ __forceinline__ void gather_warp_fp32(const InstDev* __restrict__ ins
 #ifndef GP_GATHER_MIN_BLOCKS
 #define GP_GATHER_MIN_BLOCKS 2
 #endif
+// The gathers work through a warp's slots two (FP64) or four (mixed) at a time, each group
+// a round trip to L2, so an ensemble that does not fill the chip's warps 32 to a warp is
+// handed out in shorter runs: 10,000 particles on 64^3, FP64, 29 us in runs of 32, 19 in
+// runs of 4 (48 by single lanes).
+inline int gather_run(int64_t n) {
+  constexpr int64_t kWarps = 148 * 16;   // resident
+  return n > 16 * kWarps ? 32 : (n > 8 * kWarps ? 16 : (n > 4 * kWarps ? 8 : 4));
+}
+
 template <bool kMixed>
 __global__ void __launch_bounds__(256, GP_GATHER_MIN_BLOCKS) k_gather(const InstDev* __restrict__ insts,
                                                 const PoolView* __restrict__ src_pv,
-                                                const int32_t* __restrict__ perm, int64_t n,
+                                                const int32_t* __restrict__ perm, int64_t n, int run,
                                                 double* const* __restrict__ fluid,
                                                 unsigned long long* __restrict__ ticket, Status* st) {
+  __shared__ double results[kMixed ? 1 : 8 * 6 * 32];   // one 6 x 32 block a warp (FP64 form)
   if (step_halted(st)) return;
   const int lane = threadIdx.x & 31;
   for (;;) {
     unsigned long long wt = 0;
     if (lane == 0) wt = atomicAdd(ticket, 1ull);
     const int64_t w = (int64_t)__shfl_sync(0xffffffffu, wt, 0);
-    if (w * 32 >= n) break;
-    const int64_t j = w * 32 + lane;
+    if (w * run >= n) break;
+    const int64_t j = w * run + lane;
+    const bool own = lane < run && j < n;
     int inst = -1;
     int64_t i = 0;
-    if (j < n) {
+    if (own) {
       i = perm[j];
       inst = src_pv->inst[i];
     }
@@ -720,19 +807,22 @@ __global__ void __launch_bounds__(256, GP_GATHER_MIN_BLOCKS) k_gather(const Inst
     if (inst >= 0) {
       const InstDev& I = insts[inst];
       if (stencil(I, src_pv->st[0][i], src_pv->st[1][i], src_pv->st[2][i], s)) {
-        mode = (kMixed && s.contiguous) ? 1 : 2;
+        mode = s.contiguous ? 1 : 2;
       } else {
         set_error(st, GP_EOUT_OF_GRID, (long long)src_pv->id[i], inst);
       }
     }
-    if (j < n && mode == 0) {
+    if (own && mode == 0) {
 #pragma unroll
       for (int c = 0; c < 6; ++c) fluid[c][j] = CUDART_NAN;
     }
-    if (kMixed) {
-      const int64_t b = (mode == 1) ? field_point(insts[inst], s.ix[0], s.j0 - 1, s.k0 - 1) : 0;
-      gather_warp_fp32(insts, mode, inst, b, (float)s.alfa, (float)s.beta, (float)s.gama, w * 32, fluid);
-    }
+    const int64_t b = (mode == 1) ? field_point(insts[inst], s.ix[0], s.j0 - 1, s.k0 - 1) : 0;
+    if (kMixed)
+      gather_warp_fp32(insts, mode, inst, b, (float)s.alfa, (float)s.beta, (float)s.gama, w * run, run,
+                       fluid);
+    else
+      gather_warp_fp64(insts, mode, inst, b, s.alfa, s.beta, s.gama, w * run, run,
+                       results + (threadIdx.x >> 5) * (6 * 32), fluid);
     if (mode == 2) {
       const InstDev& I = insts[inst];
       double g[6];

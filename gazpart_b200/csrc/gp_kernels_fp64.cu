@@ -15,13 +15,13 @@ template __global__ void k_integrate<false>(const InstDev *, const PoolView *, c
 template __global__ void k_integrate_fix<false>(const InstDev *, const PoolView *, const PoolView *, const PairRec *,
                                                 const unsigned long long *, int64_t, const double *const *,
                                                 uint32_t *, Status *);
-template __global__ void k_gather<false>(const InstDev *, const PoolView *, const int32_t *, int64_t,
+template __global__ void k_gather<false>(const InstDev *, const PoolView *, const int32_t *, int64_t, int,
                                          double *const *, unsigned long long *, Status *);
 
 void launch_gather_fp64(const InstDev *insts, const PoolView *pv, const int32_t *perm, int64_t n,
                       double *const *fluid, unsigned long long *ticket, Status *st, int grid, cudaStream_t s) {
   cudaMemsetAsync(ticket, 0, sizeof(unsigned long long), s);
-  k_gather<false><<<grid, 256, 0, s>>>(insts, pv, perm, n, fluid, ticket, st);
+  k_gather<false><<<grid, 256, 0, s>>>(insts, pv, perm, n, gather_run(n), fluid, ticket, st);
 }
 
 void launch_integrate_fp64(const InstDev *insts, PoolView *pv, PoolView *pv_alt, const int32_t *perm, int64_t n,
