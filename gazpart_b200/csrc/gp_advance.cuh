@@ -4,6 +4,7 @@
 #pragma once
 #include <math_constants.h>
 
+#include "gp_advance_fp64.cuh"
 #include "gp_device.cuh"
 
 namespace gp {
@@ -833,6 +834,20 @@ __global__ void __launch_bounds__(256, GP_GATHER_MIN_BLOCKS) k_gather(const Inst
   }
 }
 
+// advance_particle where the straight-line step gave up (FP64 form).  Out of line, on
+// copies, so that the state of the common path stays in registers.
+struct StepState {
+  double X[3], U[3], O[3];
+  Quat Q;
+};
+static __device__ __noinline__ int advance_particle_general(const InstDev* I, const PoolView* S, int64_t si,
+                                                            const double* fluid, StepState* s) {
+  PartConst pc;
+  load_pc(*S, si, pc);
+  MixedConst mc;
+  return advance_particle<false>(*I, pc, mc, *S, si, fluid, fluid + 3, s->X, s->U, s->O, s->Q);
+}
+
 // ADV_PARTICLE_ELLP, second half, for one particle: particle i of the source buffer is
 // advanced and written to slot j of the destination buffer with its properties, id and
 // instance (any permutation is correct: every particle carries its own record).  The
@@ -860,8 +875,18 @@ __device__ __forceinline__ void integrate_slot(const InstDev* __restrict__ insts
   // stencil out of range (reported by the gather): carried over unchanged
   if (inst >= 0 && !(uf[0] != uf[0] && wv[0] != wv[0])) {
     const InstDev& I = insts[inst];
-    if (kMixed) mixed_const(pc, I.visc, mc);
-    const int err = advance_particle<kMixed>(I, pc, mc, *S, i, uf, wv, X, U, O, Q);
+    int err = 0;
+    if (kMixed) {
+      mixed_const(pc, I.visc, mc);
+      err = advance_particle<kMixed>(I, pc, mc, *S, i, uf, wv, X, U, O, Q);
+    } else if (!advance_particle_fast(I, pc, uf, wv, X, U, O, Q)) {
+      const double fl[6] = {uf[0], uf[1], uf[2], wv[0], wv[1], wv[2]};
+      StepState s = {{X[0], X[1], X[2]}, {U[0], U[1], U[2]}, {O[0], O[1], O[2]}, Q};
+      err = advance_particle_general(&I, S, i, fl, &s);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) { X[k] = s.X[k]; U[k] = s.U[k]; O[k] = s.O[k]; }
+      Q = s.Q;
+    }
     if (err) set_error(st, err, (long long)S->id[i], inst);
     // adv_particle_new.f90:685-686: the channel wraps y and z only
     // (boundary_particle_yz.f90:44-70), the others every direction when periodic
