@@ -625,8 +625,8 @@ int enqueue_contact_response(gp_ctx *c) {
   }
   GP_TRY(mark(c, 2 * GP_PHASE_CONTACT + 1, c->stream));
   GP_TRY(mark(c, 2 * GP_PHASE_RESPONSE, c->stream));
-  launch_match(c->d_coll, c->d_counters + 1, c->cap_coll, c->d_best1, c->d_best2, c->d_matched, c->d_state,
-               c->d_status, c->stream);
+  launch_match(c->d_coll, c->d_counters + 1, c->cap_coll, c->d_best1, c->d_matched, c->d_state, c->d_status,
+               c->stream);
   launch_response(c->d_inst, c->d_pv, c->d_coll, c->d_counters + 1, c->cap_coll, c->d_state, c->d_acc,
                   c->d_counters + 2, c->d_status, 148 * 4, c->stream);
   if (c->colstats)

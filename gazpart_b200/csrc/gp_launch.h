@@ -100,7 +100,7 @@ void launch_bin_scatter(const InstDev *insts, const PoolView *pv, int64_t n, Sea
 void launch_search(const InstDev *insts, int64_t n, SearchArrays sa, PairRec *pairs, unsigned long long *npairs,
                    int64_t cap_pairs, Status *st, int grid, cudaStream_t s);
 void launch_match(const CollRec *coll, const unsigned long long *ncoll, int64_t cap_coll, unsigned long long *best1,
-                  unsigned long long *best2, int8_t *matched, int8_t *state, Status *st, cudaStream_t s);
+                  int8_t *matched, int8_t *state, Status *st, cudaStream_t s);
 void launch_field_layout(void *dst, int prec, int nx, int ny, int nz, int ncomp, int comp, const double *src,
                          int src_layout, int ghost_mode, cudaStream_t s);
 void launch_retire(const PoolView *pv, int64_t n, int inst, cudaStream_t s);

@@ -604,89 +604,106 @@ void launch_search(const InstDev *insts, int64_t n, SearchArrays sa, PairRec *pa
 // 5. lexicographically-first maximal matching of the colliding pairs
 //    (the outcome of the COLOR walk, collision_interaction.f90:190-207,397-398)
 // ---------------------------------------------------------------------------
-constexpr int kMatchThreads = 1024;
+// Rounds over the live pairs: each particle's smallest live key (A), the pairs that hold it
+// at both ends are accepted and colour their particles (B), pairs with a coloured particle
+// die and the others give their particles back (C).  A particle's smallest key is kept as
+// the index of the pair that has it, so a round takes three barriers (five with the two key
+// words kept apart).  What bounds it is the latency of the scattered accesses between two
+// barriers, so from kMatchAlone pairs on eight blocks of a cluster share the pairs, and its
+// barrier takes the place of the block's.  Measured (B200, with the response): 50,900 pairs
+// 0.88 ms in one block with five barriers -> 0.16; 3,260 pairs 0.068 alone, 0.041 shared;
+// 861 pairs 0.031 alone, 0.037 shared.
+constexpr int kMatchThreads = 1024, kMatchBlocks = 8;
+constexpr int64_t kMatchAlone = 2048;
 
-__global__ void __launch_bounds__(kMatchThreads) k_match(const CollRec *__restrict__ coll,
-                                                         const unsigned long long *__restrict__ ncoll, int64_t cap,
-                                                         unsigned long long *best1, unsigned long long *best2,
-                                                         int8_t *matched, int8_t *state, Status *st) {
-  if (step_halted(st)) return;
-  __shared__ int remaining_s[kMatchThreads / 32];
-  __shared__ int remaining;
-  const int64_t nc = (int64_t)min(*ncoll, (unsigned long long)cap);
-  const unsigned long long kMax = ~0ull;
-  for (int64_t e = threadIdx.x; e < nc; e += kMatchThreads) state[e] = 0;
-  __syncthreads();
-  bool done = (nc == 0);
-  int64_t pass = 0;
-  while (!done) {
-    for (int64_t e = threadIdx.x; e < nc; e += kMatchThreads) {
-      if (state[e] != 0) continue;
-      const CollRec &r = coll[e];
-      atomicMin(&best1[r.home], r.k1);
-      atomicMin(&best1[r.near], r.k1);
-    }
-    __syncthreads();
-    for (int64_t e = threadIdx.x; e < nc; e += kMatchThreads) {
-      if (state[e] != 0) continue;
-      const CollRec &r = coll[e];
-      if (best1[r.home] == r.k1) atomicMin(&best2[r.home], r.k2);
-      if (best1[r.near] == r.k1) atomicMin(&best2[r.near], r.k2);
-    }
-    __syncthreads();
-    for (int64_t e = threadIdx.x; e < nc; e += kMatchThreads) {
-      if (state[e] != 0) continue;
-      const CollRec &r = coll[e];
-      if (best1[r.home] == r.k1 && best2[r.home] == r.k2 && best1[r.near] == r.k1 && best2[r.near] == r.k2) {
-        state[e] = 3;   // accepted in this pass
-        matched[r.home] = 1;
-        matched[r.near] = 1;
-      }
-    }
-    __syncthreads();
-    for (int64_t e = threadIdx.x; e < nc; e += kMatchThreads) {
-      const int8_t sv = state[e];
-      if (sv != 0 && sv != 3) continue;
-      const CollRec &r = coll[e];
-      best1[r.home] = kMax; best1[r.near] = kMax;
-      best2[r.home] = kMax; best2[r.near] = kMax;
-    }
-    __syncthreads();
-    int cnt = 0;
-    for (int64_t e = threadIdx.x; e < nc; e += kMatchThreads) {
-      const int8_t sv = state[e];
-      if (sv == 3) { state[e] = 1; continue; }
-      if (sv != 0) continue;
-      const CollRec &r = coll[e];
-      if (matched[r.home] || matched[r.near]) state[e] = 2; else ++cnt;
-    }
-    cnt = __reduce_add_sync(0xffffffffu, cnt);
-    if ((threadIdx.x & 31) == 0) remaining_s[threadIdx.x >> 5] = cnt;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int t = 0;
-      for (int w = 0; w < kMatchThreads / 32; ++w) t += remaining_s[w];
-      remaining = t;
-    }
-    __syncthreads();
-    ++pass;
-    done = (remaining == 0);
-    if (!done && pass > nc + 1) {   // every pass accepts at least one pair; cannot happen
-      if (threadIdx.x == 0) set_error(st, GP_ETIMEOUT, pass);
-      done = true;
-    }
-  }
-  __syncthreads();
-  for (int64_t e = threadIdx.x; e < nc; e += kMatchThreads) {
-    const CollRec &r = coll[e];
-    matched[r.home] = 0;
-    matched[r.near] = 0;
+__device__ __forceinline__ bool key_less(const CollRec &a, const CollRec &b) {
+  return a.k1 < b.k1 || (a.k1 == b.k1 && a.k2 < b.k2);
+}
+
+// best[p] <- e if pair e's key is below that of the pair held there (~0: none)
+__device__ __forceinline__ void hold_smallest(uint32_t *best, const CollRec *coll, uint32_t e, const CollRec &r) {
+  uint32_t cur = atomicCAS(best, ~0u, e);
+  while (cur != ~0u && key_less(r, coll[cur])) {   // keys only fall, so this ends
+    const uint32_t was = atomicCAS(best, cur, e);
+    if (was == cur) break;
+    cur = was;
   }
 }
 
+__global__ void __cluster_dims__(kMatchBlocks, 1, 1) __launch_bounds__(kMatchThreads)
+    k_match(const CollRec *__restrict__ coll, const unsigned long long *__restrict__ ncoll, int64_t cap,
+            unsigned long long *best64, int8_t *matched, int8_t *state, Status *st) {
+  if (step_halted(st)) return;
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ unsigned left[2];   // live pairs after an even and an odd round (block 0's are used)
+  const int64_t nc = (int64_t)min(*ncoll, (unsigned long long)cap);
+  const bool alone = nc <= kMatchAlone;
+  if (alone && blockIdx.x != 0) return;
+  // one 32-bit index a particle, at the particle's own 64-bit word (all ones at rest)
+  uint32_t *best = reinterpret_cast<uint32_t *>(best64);
+  const int64_t first = (alone ? 0 : (int64_t)blockIdx.x * kMatchThreads) + threadIdx.x;
+  const int64_t stride = alone ? kMatchThreads : kMatchThreads * kMatchBlocks;
+  auto sync = [&]() {
+    if (alone) __syncthreads(); else cluster.sync();
+  };
+  unsigned *const left0 = cluster.map_shared_rank(left, 0);
+  if (threadIdx.x < 2) left[threadIdx.x] = 0u;
+  for (int64_t e = first; e < nc; e += stride) state[e] = 0;
+  sync();
+  bool live = nc > 0;
+  for (int64_t round = 0; live; ++round) {
+    for (int64_t e = first; e < nc; e += stride) {
+      if (state[e] != 0) continue;
+      const CollRec &r = coll[e];
+      hold_smallest(best + 2 * (int64_t)r.home, coll, (uint32_t)e, r);
+      hold_smallest(best + 2 * (int64_t)r.near, coll, (uint32_t)e, r);
+    }
+    sync();
+    if (blockIdx.x == 0 && threadIdx.x == 0) left[(round + 1) & 1] = 0u;
+    for (int64_t e = first; e < nc; e += stride) {
+      if (state[e] != 0) continue;
+      const CollRec &r = coll[e];
+      if (__ldcg(best + 2 * (int64_t)r.home) == (uint32_t)e && __ldcg(best + 2 * (int64_t)r.near) == (uint32_t)e) {
+        state[e] = 1;
+        __stcg(matched + r.home, (int8_t)1);
+        __stcg(matched + r.near, (int8_t)1);
+      }
+    }
+    sync();
+    unsigned cnt = 0;
+    for (int64_t e = first; e < nc; e += stride) {
+      if (state[e] != 0) continue;
+      const CollRec &r = coll[e];
+      if (__ldcg(matched + r.home) || __ldcg(matched + r.near)) {
+        state[e] = 2;
+      } else {
+        __stcg(best + 2 * (int64_t)r.home, ~0u);
+        __stcg(best + 2 * (int64_t)r.near, ~0u);
+        ++cnt;
+      }
+    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(left0 + (round & 1), cnt);
+    sync();
+    live = *(volatile unsigned *)(left0 + (round & 1)) != 0u;
+    if (live && round > nc) {   // every round accepts at least one pair; cannot happen
+      if (first == 0) set_error(st, GP_ETIMEOUT, round);
+      live = false;
+    }
+  }
+  for (int64_t e = first; e < nc; e += stride) {
+    const CollRec &r = coll[e];
+    __stcg(best + 2 * (int64_t)r.home, ~0u);
+    __stcg(best + 2 * (int64_t)r.near, ~0u);
+    __stcg(matched + r.home, (int8_t)0);
+    __stcg(matched + r.near, (int8_t)0);
+  }
+  if (!alone) cluster.sync();   // block 0's counters stay until every block has read them
+}
+
 void launch_match(const CollRec *coll, const unsigned long long *ncoll, int64_t cap_coll, unsigned long long *best1,
-                  unsigned long long *best2, int8_t *matched, int8_t *state, Status *st, cudaStream_t s) {
-  k_match<<<1, kMatchThreads, 0, s>>>(coll, ncoll, cap_coll, best1, best2, matched, state, st);
+                  int8_t *matched, int8_t *state, Status *st, cudaStream_t s) {
+  k_match<<<kMatchBlocks, kMatchThreads, 0, s>>>(coll, ncoll, cap_coll, best1, matched, state, st);
 }
 
 // ---------------------------------------------------------------------------
