@@ -275,7 +275,7 @@ int class_props(gp_ctx *c, int ig, int idp, double pc[kNConst]) {
 }
 
 void free_search(gp_ctx *c) {
-  dfree(c->sa.cell_count); dfree(c->sa.cell_start); dfree(c->sa.cell_fill); dfree(c->sa.cell_rmax);
+  dfree(c->sa.cell_count); dfree(c->sa.cell_start); dfree(c->sa.cell_rmax);
   dfree(c->d_scan_tmp);
   c->ncells_cap = 0;
 }
@@ -288,9 +288,7 @@ void free_pool(gp_ctx *c) {
     dfree(c->d_instof[b]);
   }
   for (auto &p : c->d_fluid) dfree(p);
-  dfree(c->sa.cell_of); dfree(c->sa.sorted); dfree(c->sa.sx); dfree(c->sa.sy); dfree(c->sa.sz); dfree(c->sa.sr);
-  dfree(c->sa.sbox); dfree(c->sa.sinst); dfree(c->sa.sid);
-  dfree(c->sa.spk); dfree(c->sa.sex); dfree(c->sa.sey); dfree(c->sa.sez); dfree(c->sa.sa2); dfree(c->sa.sb2);
+  dfree(c->sa.cell_of); dfree(c->sa.sorted); dfree(c->sa.spk);
   dfree(c->d_best1); dfree(c->d_best2); dfree(c->d_matched);
   dfree(c->d_pairs); dfree(c->d_coll); dfree(c->d_state); dfree(c->d_acc);
   dfree(c->d_mark);
@@ -358,11 +356,7 @@ int alloc_pool(gp_ctx *c, int64_t cap) {
   }
   for (auto &p : c->d_fluid) GP_TRY(dalloc(&p, cap));   // interpolated field at each particle
   SearchArrays &sa = c->sa;
-  GP_TRY(dalloc(&sa.cell_of, cap)); GP_TRY(dalloc(&sa.sorted, cap));
-  GP_TRY(dalloc(&sa.sx, cap)); GP_TRY(dalloc(&sa.sy, cap)); GP_TRY(dalloc(&sa.sz, cap)); GP_TRY(dalloc(&sa.sr, cap));
-  GP_TRY(dalloc(&sa.sbox, cap)); GP_TRY(dalloc(&sa.sinst, cap)); GP_TRY(dalloc(&sa.sid, cap));
-  GP_TRY(dalloc(&sa.spk, cap)); GP_TRY(dalloc(&sa.sex, cap)); GP_TRY(dalloc(&sa.sey, cap)); GP_TRY(dalloc(&sa.sez, cap));
-  GP_TRY(dalloc(&sa.sa2, cap)); GP_TRY(dalloc(&sa.sb2, cap));
+  GP_TRY(dalloc(&sa.cell_of, cap)); GP_TRY(dalloc(&sa.sorted, cap)); GP_TRY(dalloc(&sa.spk, cap));
   GP_TRY(dalloc(&c->d_best1, cap)); GP_TRY(dalloc(&c->d_best2, cap)); GP_TRY(dalloc(&c->d_matched, cap));
   GP_CK(cudaMemsetAsync(c->d_best1, 0xFF, cap * sizeof(unsigned long long), c->stream));
   GP_CK(cudaMemsetAsync(c->d_best2, 0xFF, cap * sizeof(unsigned long long), c->stream));
@@ -430,6 +424,8 @@ int setup_grids(InstDev &I, double max_emaj, double rmax, double rsmall, int64_t
   I.hfx = I.lx / I.nfx; I.hfy = I.ly / I.nfy; I.hfz = I.lz / I.nfz;
   I.rmax = rmax;
   I.rcut = 0.5 * std::min(I.hfx, std::min(I.hfy, I.hfz)) / (1.0 + 1.0e-6);
+  I.ihfx = 1.0 / I.hfx; I.ihfy = 1.0 / I.hfy; I.ihfz = 1.0 / I.hfz;
+  I.slack = (float)(2e-6 * std::max(I.lx, std::max(I.ly, I.lz)));
   I.cell_begin = cell_begin;
   const int64_t ncells = (int64_t)I.nfx * I.nfy * I.nfz;
   if (ncells >= (int64_t(1) << 31) - 2) return GP_EBADARG;
@@ -442,8 +438,8 @@ int alloc_cells(gp_ctx *c, int64_t ncells) {
     free_search(c);
     GP_TRY(dalloc(&c->sa.cell_count, ncells + 1));
     GP_TRY(dalloc(&c->sa.cell_start, ncells + 1));
-    GP_TRY(dalloc(&c->sa.cell_fill, ncells + 1));
     GP_TRY(dalloc(&c->sa.cell_rmax, ncells + 1));
+    GP_CK(cudaMemsetAsync(c->sa.cell_count, 0, (ncells + 1) * sizeof(int32_t), c->stream));
     GP_TRY(dalloc(&c->d_scan_tmp, (size_t)scan_block_sums_size(ncells)));
     c->ncells_cap = ncells;
   }
@@ -561,12 +557,9 @@ int enqueue_advance(gp_ctx *c) {
 // Binning of the search grid (also the cell order the next advance moves to).
 int enqueue_bin(gp_ctx *c) {
   SearchArrays sa = c->sa;
-  GP_CK(cudaMemsetAsync(sa.cell_count, 0, (c->ncells + 1) * sizeof(int32_t), c->stream));
-  GP_CK(cudaMemsetAsync(sa.cell_fill, 0, (c->ncells + 1) * sizeof(int32_t), c->stream));
-  GP_CK(cudaMemsetAsync(sa.cell_rmax, 0, (c->ncells + 1) * sizeof(float), c->stream));
   GP_CK(cudaMemsetAsync(c->d_counters, 0, 6 * sizeof(unsigned long long), c->stream));
   launch_bin_count(c->d_inst, c->d_pv, c->n_slots, sa, c->d_status, c->tune[GP_TUNE_BIN], c->stream);
-  launch_scan(sa.cell_count, sa.cell_start, c->ncells, c->d_scan_tmp, c->stream);
+  launch_scan(sa.cell_count, sa.cell_start, c->ncells, c->d_scan_tmp, sa.cell_rmax, c->stream);
   launch_bin_scatter(c->d_inst, c->d_pv, c->n_slots, sa, c->d_status, c->tune[GP_TUNE_BIN], c->stream);
   GP_CK(cudaGetLastError());
   return GP_OK;
@@ -581,7 +574,7 @@ int enqueue_bin_search(gp_ctx *c, bool flag = false) {
   GP_TRY(mark(c, 2 * GP_PHASE_BIN + 1, c->stream));
   GP_TRY(mark(c, 2 * GP_PHASE_SEARCH, c->stream));
   // a step with more candidates than either pair buffer holds halts after the search
-  launch_search(c->d_inst, c->n, sa, c->d_pairs, c->d_counters + 0, std::min(c->cap_pairs, c->cap_coll),
+  launch_search(c->d_inst, c->d_pv, c->n, sa, c->d_pairs, c->d_counters + 0, std::min(c->cap_pairs, c->cap_coll),
                 c->d_status, c->tune[GP_TUNE_SEARCH], c->stream);
   // The contact queue's order: the pairs in decreasing predicted length, from the
   // particles' record of the last collision phase, which is then cleared for this one.

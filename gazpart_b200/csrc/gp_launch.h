@@ -93,11 +93,12 @@ void launch_iota(int32_t *a, int64_t n, cudaStream_t s);
 // --- gp_search.cu ---
 void launch_bin_count(const InstDev *insts, const PoolView *pv, int64_t n, SearchArrays sa, Status *st, int grid,
                       cudaStream_t s);
-void launch_scan(const int32_t *in, int32_t *out, int64_t n, int32_t *block_sums, cudaStream_t s);
+// (clears clear[0..n) on the way)
+void launch_scan(const int32_t *in, int32_t *out, int64_t n, int32_t *block_sums, float *clear, cudaStream_t s);
 int64_t scan_block_sums_size(int64_t n);
 void launch_bin_scatter(const InstDev *insts, const PoolView *pv, int64_t n, SearchArrays sa, Status *st, int grid,
                         cudaStream_t s);
-void launch_search(const InstDev *insts, int64_t n, SearchArrays sa, PairRec *pairs, unsigned long long *npairs,
+void launch_search(const InstDev *insts, const PoolView *pv, int64_t n, SearchArrays sa, PairRec *pairs, unsigned long long *npairs,
                    int64_t cap_pairs, Status *st, int grid, cudaStream_t s);
 void launch_match(const CollRec *coll, const unsigned long long *ncoll, int64_t cap_coll, unsigned long long *best1,
                   int8_t *matched, int8_t *state, Status *st, cudaStream_t s);

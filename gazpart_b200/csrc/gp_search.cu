@@ -54,13 +54,23 @@ __device__ __forceinline__ int wrap_delta(int d, int n, bool periodic) {
 }
 
 
-// ---------------------------------------------------------------------------
 // 1. search-grid cell of every particle (counting pass)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int cell_coord(double v, double h, int n) {
-  const double f = v / h;
+__device__ __forceinline__ int cell_coord(double v, double ih, int n) {
+  const double f = v * ih;
   int c = (f >= 0.0) ? (f < (double)n ? (int)f : n - 1) : 0;
   return c;
+}
+
+// First cell of the row (cy, cz); cells are numbered x-fastest.
+__device__ __forceinline__ int32_t cell_row(const InstDev &I, int cy, int cz) {
+  return (int32_t)I.cell_begin + (cz * I.nfy + cy) * I.nfx;
+}
+__device__ __forceinline__ void cell_coords(const InstDev &I, int32_t cell, int &cx, int &cy, int &cz) {
+  const int l = cell - (int32_t)I.cell_begin, t = l / I.nfx;
+  cx = l - t * I.nfx;
+  cz = t / I.nfy;
+  cy = t - cz * I.nfy;
 }
 
 __global__ void k_bin_count(const InstDev *__restrict__ insts, const PoolView *__restrict__ pv, int64_t n,
@@ -75,10 +85,10 @@ __global__ void k_bin_count(const InstDev *__restrict__ insts, const PoolView *_
       const int inst = P.inst[i];
       if (inst >= 0) {
         const InstDev &I = insts[inst];
-        const int cx = cell_coord(P.st[0][i], I.hfx, I.nfx);
-        const int cy = cell_coord(P.st[1][i], I.hfy, I.nfy);
-        const int cz = cell_coord(P.st[2][i], I.hfz, I.nfz);
-        c = (int32_t)(I.cell_begin + ((int64_t)cz * I.nfy + cy) * I.nfx + cx);
+        const int cx = cell_coord(P.st[0][i], I.ihfx, I.nfx);
+        const int cy = cell_coord(P.st[1][i], I.ihfy, I.nfy);
+        const int cz = cell_coord(P.st[2][i], I.ihfz, I.nfz);
+        c = cell_row(I, cy, cz) + cx;
       }
       sa.cell_of[i] = c;
     }
@@ -101,7 +111,7 @@ void launch_bin_count(const InstDev *insts, const PoolView *pv, int64_t n, Searc
 constexpr int kScanThreads = 512, kScanPer = 4, kScanBlock = kScanThreads * kScanPer;
 
 __global__ void k_scan_block(const int32_t *__restrict__ in, int32_t *__restrict__ out, int64_t n,
-                             int32_t *__restrict__ sums) {
+                             int32_t *__restrict__ sums, float *__restrict__ clear) {
   __shared__ int32_t warp_tot[kScanThreads / 32];
   const int64_t base = (int64_t)blockIdx.x * kScanBlock + (int64_t)threadIdx.x * kScanPer;
   int32_t v[kScanPer];
@@ -138,7 +148,10 @@ __global__ void k_scan_block(const int32_t *__restrict__ in, int32_t *__restrict
 #pragma unroll
   for (int k = 0; k < kScanPer; ++k) {
     const int64_t idx = base + k;
-    if (idx < n) out[idx] = v[k] + excl;
+    if (idx < n) {
+      out[idx] = v[k] + excl;
+      if (clear != nullptr) clear[idx] = 0.f;
+    }
   }
   if (threadIdx.x == kScanThreads - 1 && sums != nullptr) sums[blockIdx.x] = excl + run;
 }
@@ -161,16 +174,16 @@ int64_t scan_block_sums_size(int64_t n) {
 }
 
 // out[0..n] = exclusive scan of in[0..n-1], out[n] = total.  in[n] must be readable
-// as zero (the caller allocates n+1 counters).
-void launch_scan(const int32_t *in, int32_t *out, int64_t n, int32_t *tmp, cudaStream_t s) {
+// as zero (the caller allocates n+1 counters, and n+1 values of clear).
+void launch_scan(const int32_t *in, int32_t *out, int64_t n, int32_t *tmp, float *clear, cudaStream_t s) {
   const int64_t m = n + 1;
   const int64_t b1 = nblocks(m), b2 = nblocks(b1), b3 = nblocks(b2);
   int32_t *s1 = tmp, *s1x = s1 + b1, *s2 = s1x + b1, *s2x = s2 + b2, *s3 = s2x + b2;
-  k_scan_block<<<(unsigned)b1, kScanThreads, 0, s>>>(in, out, m, s1);
+  k_scan_block<<<(unsigned)b1, kScanThreads, 0, s>>>(in, out, m, s1, clear);
   if (b1 > 1) {
-    k_scan_block<<<(unsigned)b2, kScanThreads, 0, s>>>(s1, s1x, b1, s2);
+    k_scan_block<<<(unsigned)b2, kScanThreads, 0, s>>>(s1, s1x, b1, s2, nullptr);
     if (b2 > 1) {
-      k_scan_block<<<(unsigned)b3, kScanThreads, 0, s>>>(s2, s2x, b2, s3);   // b3 == 1 for n < 8.6e9
+      k_scan_block<<<(unsigned)b3, kScanThreads, 0, s>>>(s2, s2x, b2, s3, nullptr);   // b3 == 1 for n < 8.6e9
       k_scan_add<<<(unsigned)b2, kScanThreads, 0, s>>>(s1x, b1, s2x);
     }
     k_scan_add<<<(unsigned)b1, kScanThreads, 0, s>>>(out, m, s1x);
@@ -178,8 +191,29 @@ void launch_scan(const int32_t *in, int32_t *out, int64_t n, int32_t *tmp, cudaS
 }
 
 // ---------------------------------------------------------------------------
-// 3. scatter into cell order + reference box ids (collision_detection_connectivity.f90:74-89)
+// 3. scatter into cell order, out-of-grid check (collision_detection_connectivity.f90:74-89)
 // ---------------------------------------------------------------------------
+// 0-based coordinate of v in the reference's box grid, or -1 outside it.
+__device__ __forceinline__ int box_coord(double v, double vmin, double edge, int nbox) {
+  const double f = (v - vmin) / edge;
+  if (!(f > -1.0 && f < 2.0e9)) return -1;
+  const int k = (int)f + 1;
+  return (k >= 1 && k <= nbox) ? k - 1 : -1;
+}
+// Whether box_coord has a box for v, without its division well inside the grid.
+__device__ __forceinline__ bool in_boxes(double v, double vmin, double edge, int nbox) {
+  const double d = v - vmin;
+  return (d >= 0.0 && d <= (double)nbox * edge * (1.0 - 1e-9)) || box_coord(v, vmin, edge, nbox) >= 0;
+}
+
+// The counting pass's counts are taken back to zero here, one place after the other, so
+// that the next binning finds them clear.  Only what nearly every candidate of the search
+// is judged by goes into sorted order (20 bytes a particle); the few candidates that pass
+// read the pool.  What bounds it is the scattered traffic: with sixteen sorted columns
+// (112 bytes written, 100 read) and three arrays of cells cleared by themselves the whole
+// binning took 1.07 ms at 16.8 M particles, with these two 0.65 (B200).  Numbering the
+// cells in bricks of 4 x 4 x 8, 4 x 4 x 4 or 2 x 2 x 8 for the gather's sake left the
+// gather as it was (3.22 ms each) and took 0.04 more in the search.
 __global__ void k_bin_scatter(const InstDev *__restrict__ insts, const PoolView *__restrict__ pv, int64_t n,
                               SearchArrays sa, Status *st) {
   if (step_halted(st)) return;
@@ -191,44 +225,32 @@ __global__ void k_bin_scatter(const InstDev *__restrict__ insts, const PoolView 
     const int32_t c = (i < n) ? sa.cell_of[i] : -1;
     const unsigned peers = __match_any_sync(0xffffffffu, c);
     const int leader = __ffs(peers) - 1;
+    double x = 0.0, y = 0.0, z = 0.0;
+    float small = 0.f, w = 0.f;
+    if (c >= 0) {
+      const int inst = P.inst[i];
+      const InstDev &I = insts[inst];
+      x = P.st[0][i]; y = P.st[1][i]; z = P.st[2][i];
+      const double rb = fmax(P.pc[0][i], P.pc[1][i]);
+      // w carries the bounding radius, negated for particles above the small-particle cut
+      w = rb > I.rcut ? -(float)rb : (float)rb;
+      if (rb <= I.rcut) small = __double2float_ru(rb);   // a float rounded up bounds the radius
+      if (!(in_boxes(x, I.xminbox, I.dxbox, I.nxbox) && in_boxes(y, I.yminbox, I.dybox, I.nybox) &&
+            in_boxes(z, I.zminbox, I.dzbox, I.nzbox)))
+        set_error(st, GP_EOUT_OF_GRID, (long long)P.id[i], inst);
+    }
+    // non-negative floats order like their bits
+    const unsigned most = __reduce_max_sync(peers, (unsigned)__float_as_int(small));
     int base = 0;
-    if (c >= 0 && lane == leader) base = atomicAdd(&sa.cell_fill[c], __popc(peers));
+    if (c >= 0 && lane == leader) {
+      base = atomicSub(&sa.cell_count[c], __popc(peers)) - __popc(peers);
+      if (most != 0u) atomicMax(reinterpret_cast<int *>(sa.cell_rmax) + c, (int)most);
+    }
     base = __shfl_sync(0xffffffffu, base, leader);
     if (c < 0) continue;
     const int pos = sa.cell_start[c] + base + __popc(peers & ((1u << lane) - 1u));
-    const int inst = P.inst[i];
-    const InstDev &I = insts[inst];
-    const double x = P.st[0][i], y = P.st[1][i], z = P.st[2][i];
     sa.sorted[pos] = (int32_t)i;
-    sa.sx[pos] = x;
-    sa.sy[pos] = y;
-    sa.sz[pos] = z;
-    const double ea = P.pc[0][i], eb = P.pc[1][i];
-    sa.sr[pos] = fmax(ea, eb);
-    // w carries the bounding radius, negated for particles above the small-particle cut
-    const double rb = fmax(ea, eb);
-    sa.spk[pos] = make_float4((float)x, (float)y, (float)z, rb > I.rcut ? -(float)rb : (float)rb);
-    // a float rounded up bounds the radius; non-negative floats order like their bits
-    if (rb <= I.rcut) atomicMax(reinterpret_cast<int *>(sa.cell_rmax) + c, __float_as_int(__double2float_ru(rb)));
-    sa.sa2[pos] = ea * ea;
-    sa.sb2[pos] = eb * eb;
-    {
-      const double q0 = P.st[6][i], q1 = P.st[7][i], q2 = P.st[8][i], q3 = P.st[9][i];
-      sa.sex[pos] = 1.0 - 2.0 * (q2 * q2 + q3 * q3);
-      sa.sey[pos] = 2.0 * (q1 * q2 + q0 * q3);
-      sa.sez[pos] = 2.0 * (q1 * q3 - q0 * q2);
-    }
-    sa.sinst[pos] = inst;
-    sa.sid[pos] = P.id[i];
-    const double fx = (x - I.xminbox) / I.dxbox, fy = (y - I.yminbox) / I.dybox, fz = (z - I.zminbox) / I.dzbox;
-    long long box = -1;
-    if (fx > -1.0 && fx < 2.0e9 && fy > -1.0 && fy < 2.0e9 && fz > -1.0 && fz < 2.0e9) {
-      const int i0 = (int)fx + 1, j0 = (int)fy + 1, k0 = (int)fz + 1;
-      if (i0 >= 1 && i0 <= I.nxbox && j0 >= 1 && j0 <= I.nybox && k0 >= 1 && k0 <= I.nzbox)
-        box = (long long)(i0 - 1) | ((long long)(j0 - 1) << 21) | ((long long)(k0 - 1) << 42);
-    }
-    if (box < 0) set_error(st, GP_EOUT_OF_GRID, (long long)P.id[i], P.inst[i]);
-    sa.sbox[pos] = box;
+    sa.spk[pos] = make_float4((float)x, (float)y, (float)z, w);
   }
 }
 
@@ -263,19 +285,21 @@ __device__ __forceinline__ void emit_pair(PairRec *pairs, unsigned long long *np
 }
 
 // A home particle as the conservative float test of its candidates reads it: position,
-// bounding radius, its instance's box lengths and x periodicity (32 bytes).
+// bounding radius, its instance's box lengths, the slack with the sign of x periodicity
+// (32 bytes).
 struct HomeF {
-  float x, y, z, r, lx, ly, lz;
-  int perx;
+  float x, y, z, r, lx, ly, lz, slack;
 };
 
-__device__ __forceinline__ HomeF home_f(const InstDev &I, double x, double y, double z, double r) {
-  return {(float)x, (float)y, (float)z, (float)r, (float)I.lx, (float)I.ly, (float)I.lz, I.periodicity != 0};
+__device__ __forceinline__ HomeF home_f(const InstDev &I, const float4 p) {
+  return {p.x, p.y, p.z, fabsf(p.w), (float)I.lx, (float)I.ly, (float)I.lz,
+          I.periodicity != 0 ? I.slack : -I.slack};
 }
 
 // The conservative float test of candidate qs (sorted position) against a home at sorted
-// position s: |float - double| distance error < 2e-6, slack 1e-5.  Nearly every
-// candidate of the sweep fails it, so it reads only the candidate's float record.
+// position s: rounding moves the float distance by less than 7e-7 of the largest box
+// length, the slack is 2e-6 of it.  Nearly every candidate of the sweep fails it, so it
+// reads only the candidate's float record.
 // kLarge: the home particle is above the cut and sweeps a full stencil; it takes every
 // small candidate and the large ones that follow it in sorted order.  Otherwise the home
 // particle is small, sweeps the half stencil and leaves large candidates to them.
@@ -283,31 +307,47 @@ template <bool kLarge>
 __device__ __forceinline__ bool near_float(const float4 c, int32_t qs, int32_t s, const HomeF &h) {
   if (c.w < 0.f && (!kLarge || qs <= s)) return false;
   float fx = c.x - h.x, fy = c.y - h.y, fz = c.z - h.z;
-  if (h.perx && fabsf(fx) > 0.5f * h.lx) fx = fx - copysignf(h.lx, fx);
+  if (h.slack > 0.f && fabsf(fx) > 0.5f * h.lx) fx = fx - copysignf(h.lx, fx);
   if (fabsf(fy) > 0.5f * h.ly) fy = fy - copysignf(h.ly, fy);
   if (fabsf(fz) > 0.5f * h.lz) fz = fz - copysignf(h.lz, fz);
-  const float rf = h.r + fabsf(c.w) + 1.0e-5f;
+  const float rf = h.r + fabsf(c.w) + fabsf(h.slack);
   return fx * fx + fy * fy + fz * fz <= rf * rf;
 }
 
-// One candidate (s, qs) of the sweep that passed near_float: FP64 bounding-sphere test,
-// centre-line separation test, reference box adjacency, then emission with the
-// reference's ordering keys.
-struct SearchHome {
-  double xp, yp, zp, rp;
-  long long bp;
-  int32_t s, pslot, idp;
-  bool perx;
+// What the exact tests of a pair take of one particle, from the pool: position, squared
+// semi-axes and bounding radius, symmetry axis in the lab frame (first column of R(q)).
+struct PairEnd {
+  double x, y, z, r, a2, b2, ex, ey, ez;
 };
+__device__ __forceinline__ PairEnd pair_end(const PoolView &P, int32_t i) {
+  PairEnd e;
+  e.x = P.st[0][i]; e.y = P.st[1][i]; e.z = P.st[2][i];
+  const double ea = P.pc[0][i], eb = P.pc[1][i];
+  const double q0 = P.st[6][i], q1 = P.st[7][i], q2 = P.st[8][i], q3 = P.st[9][i];
+  e.r = fmax(ea, eb);
+  e.a2 = ea * ea;
+  e.b2 = eb * eb;
+  e.ex = 1.0 - 2.0 * (q2 * q2 + q3 * q3);
+  e.ey = 2.0 * (q1 * q2 + q0 * q3);
+  e.ez = 2.0 * (q1 * q3 - q0 * q2);
+  return e;
+}
 
-__device__ __forceinline__ void search_candidate(const InstDev &I, const SearchArrays &sa, const SearchHome &h,
-                                                 int32_t qs, PairRec *pairs, unsigned long long *npairs,
-                                                 int64_t cap, Status *st) {
-  double dx = sa.sx[qs] - h.xp, dy = sa.sy[qs] - h.yp, dz = sa.sz[qs] - h.zp;
-  if (h.perx && fabs(dx) > I.lx / 2) dx = dx - copysign(I.lx, dx);
+// One candidate (sorted positions s, qs) of the sweep that passed near_float: FP64
+// bounding-sphere test, centre-line separation test, reference box adjacency, then emission
+// with the reference's ordering keys.
+__device__ __forceinline__ void search_candidate(const InstDev *__restrict__ insts, const PoolView &P,
+                                                 const SearchArrays &sa, int32_t s, int32_t qs, PairRec *pairs,
+                                                 unsigned long long *npairs, int64_t cap, Status *st) {
+  const int32_t pslot = sa.sorted[s], qslot = sa.sorted[qs];
+  const InstDev &I = insts[P.inst[pslot]];
+  const bool perx = I.periodicity != 0;
+  const PairEnd p = pair_end(P, pslot), q = pair_end(P, qslot);
+  double dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+  if (perx && fabs(dx) > I.lx / 2) dx = dx - copysign(I.lx, dx);
   if (fabs(dy) > I.ly / 2.) dy = dy - copysign(I.ly, dy);
   if (fabs(dz) > I.lz / 2.) dz = dz - copysign(I.lz, dz);
-  const double rr = (h.rp + sa.sr[qs]) * (1.0 + 1e-9);
+  const double rr = (p.r + q.r) * (1.0 + 1e-9);
   const double d2 = dx * dx + dy * dy + dz * dz;
   if (d2 > rr * rr) return;
   // Support-function test along the centre line: for unit d, the extent of a
@@ -317,49 +357,43 @@ __device__ __forceinline__ void search_candidate(const InstDev &I, const SearchA
   if (d2 > 0.0) {
     const double dist = sqrt(d2), inv = 1.0 / dist;
     const double ux = dx * inv, uy = dy * inv, uz = dz * inv;
-    const double cp = sa.sex[h.s] * ux + sa.sey[h.s] * uy + sa.sez[h.s] * uz;
-    const double cq = sa.sex[qs] * ux + sa.sey[qs] * uy + sa.sez[qs] * uz;
-    const double hp = sqrt(fmax(sa.sb2[h.s] + (sa.sa2[h.s] - sa.sb2[h.s]) * cp * cp, 0.0));
-    const double hq = sqrt(fmax(sa.sb2[qs] + (sa.sa2[qs] - sa.sb2[qs]) * cq * cq, 0.0));
+    const double cp = p.ex * ux + p.ey * uy + p.ez * uz;
+    const double cq = q.ex * ux + q.ey * uy + q.ez * uz;
+    const double hp = sqrt(fmax(p.b2 + (p.a2 - p.b2) * cp * cp, 0.0));
+    const double hq = sqrt(fmax(q.b2 + (q.a2 - q.b2) * cq * cq, 0.0));
     if (hp + hq < dist * (1.0 - 1e-9)) return;
   }
   atomicAdd(&st->n_near, 1ull);
   // reference adjacency of the two boxes (collision_box_connectivity.f90)
-  const long long bp = h.bp, bq = sa.sbox[qs];
-  if (bp < 0 || bq < 0) return;   // already reported as out of grid
-  const int pi = (int)(bp & 0x1FFFFF), pj = (int)((bp >> 21) & 0x1FFFFF), pk = (int)(bp >> 42);
-  const int qi = (int)(bq & 0x1FFFFF), qj = (int)((bq >> 21) & 0x1FFFFF), qk = (int)(bq >> 42);
-  const int di = wrap_delta(qi - pi, I.nxbox, h.perx);
+  const int pi = box_coord(p.x, I.xminbox, I.dxbox, I.nxbox), pj = box_coord(p.y, I.yminbox, I.dybox, I.nybox);
+  const int pk = box_coord(p.z, I.zminbox, I.dzbox, I.nzbox);
+  const int qi = box_coord(q.x, I.xminbox, I.dxbox, I.nxbox), qj = box_coord(q.y, I.yminbox, I.dybox, I.nybox);
+  const int qk = box_coord(q.z, I.zminbox, I.dzbox, I.nzbox);
+  if ((pi | pj | pk | qi | qj | qk) < 0) return;   // already reported as out of grid
+  const int di = wrap_delta(qi - pi, I.nxbox, perx);
   const int dj = wrap_delta(qj - pj, I.nybox, true);
   const int dk = wrap_delta(qk - pk, I.nzbox, true);
   if (di < -1 || di > 1 || dj < -1 || dj > 1 || dk < -1 || dk > 1) return;
-  const int32_t idq = sa.sid[qs];
+  const int32_t idp = P.id[pslot], idq = P.id[qslot];
   PairRec r;
   int slot;
-  long long hb;
   bool home_is_p;
   if (di == 0 && dj == 0 && dk == 0) {
     slot = 0;
-    home_is_p = h.idp < idq;
-    hb = bp;
+    home_is_p = idp < idq;
   } else {
     const int idx = (di + 1) * 9 + (dj + 1) * 3 + (dk + 1);
     slot = c_fwd_slot[idx];
-    if (slot > 0) {
-      home_is_p = true;
-      hb = bp;
-    } else {
-      slot = c_fwd_slot[26 - idx];
-      home_is_p = false;
-      hb = bq;
-    }
+    home_is_p = slot > 0;
+    if (!home_is_p) slot = c_fwd_slot[26 - idx];
   }
-  const int hi = (int)(hb & 0x1FFFFF), hj = (int)((hb >> 21) & 0x1FFFFF), hk = (int)(hb >> 42);
+  // the home's box (both particles' box where slot = 0)
+  const int hi = home_is_p ? pi : qi, hj = home_is_p ? pj : qj, hk = home_is_p ? pk : qk;
   const unsigned long long ijk =
       (unsigned long long)(hi + 1) + (unsigned long long)hj * I.nxbox + (unsigned long long)hk * I.nxbox * I.nybox;
-  const int32_t idh = home_is_p ? h.idp : idq, idn = home_is_p ? idq : h.idp;
-  r.home = home_is_p ? h.pslot : sa.sorted[qs];
-  r.near = home_is_p ? sa.sorted[qs] : h.pslot;
+  const int32_t idh = home_is_p ? idp : idq, idn = home_is_p ? idq : idp;
+  r.home = home_is_p ? pslot : qslot;
+  r.near = home_is_p ? qslot : pslot;
   r.k1 = ijk;
   r.k2 = ((unsigned long long)idh << 34) | ((unsigned long long)slot << 30) | (unsigned long long)idn;
   emit_pair(pairs, npairs, cap, r, sa.mark, st);
@@ -367,53 +401,19 @@ __device__ __forceinline__ void search_candidate(const InstDev &I, const SearchA
 
 __device__ __forceinline__ int wrap_cell(int c, int n) { return c < 0 ? c + n : (c >= n ? c - n : c); }
 
-// Cells [lo, hi] of one x-row as at most two contiguous ranges of sorted particles
-// (periodic x wraps, otherwise the row is clipped).  lo >= -nfx and hi < 2 nfx.
-struct RowRanges {
-  int32_t a0, a1, b0, b1;
-};
-__device__ __forceinline__ RowRanges row_ranges(const SearchArrays &sa, int64_t base, int nfx, int lo, int hi,
-                                                bool perx) {
-  RowRanges r = {0, 0, 0, 0};
-  if (hi - lo + 1 >= nfx && perx) {
-    r.a0 = sa.cell_start[base];
-    r.a1 = sa.cell_start[base + nfx];
-    return r;
-  }
-  if (lo < 0) {
-    if (perx) { r.b0 = sa.cell_start[base + nfx + lo]; r.b1 = sa.cell_start[base + nfx]; }
-    lo = 0;
-  }
-  if (hi >= nfx) {
-    if (perx) { r.b0 = sa.cell_start[base]; r.b1 = sa.cell_start[base + hi - nfx + 1]; }
-    hi = nfx - 1;
-  }
-  if (lo <= hi) {
-    r.a0 = sa.cell_start[base + lo];
-    r.a1 = sa.cell_start[base + hi + 1];
-  }
-  return r;
-}
-
 // Pair search over the search grid.  The cell edge is at least twice the cut radius,
 // so two small particles (bounding radius <= cut) can only meet in the same or an
 // adjacent cell; a small particle sweeps the half stencil of its cell: the 13 forward
 // neighbours that follow it in (z, y, x) order, (cx+1, cy, cz), the three cells
 // cx-1..cx+1 of row (cy+1, cz) and the nine of layer cz+1.  Cells are numbered
 // x-fastest, so these are five x-rows, each one or two contiguous ranges of sorted
-// particles; the home cell is swept from the next sorted particle on.  A large particle
-// (radius above the cut, rare) sweeps every cell within its radius plus the largest
-// radius.  Every pair is visited exactly once.
+// particles; the home cell is swept from the next sorted particle on.  A large particle (radius above the
+// cut, rare) sweeps every cell within its radius plus the largest radius.  Every pair is
+// visited exactly once.
 #ifndef GP_SEARCH_MIN_BLOCKS
 #define GP_SEARCH_MIN_BLOCKS 4
 #endif
 
-// A home particle's data, kept in shared memory for the lanes that test its candidates.
-struct HomeRec {
-  double xp, yp, zp, rp;
-  long long bp;
-  int32_t s, pslot, idp, inst;
-};
 constexpr int kSearchThreads = 256;
 constexpr int kMaxRanges = 10;   // 5 rows, each at most two contiguous ranges
 
@@ -423,20 +423,25 @@ constexpr int kMaxRanges = 10;   // 5 rows, each at most two contiguous ranges
 // candidates together, 32 at a time: candidate idx of the warp's concatenated lists goes
 // to lane idx mod 32, which looks up the owning home and range in shared memory.  Lanes
 // stay busy however unevenly the candidates fall among the homes.  Homes above the cut
-// radius sweep their wide stencil afterwards, each on its own lane.
+// radius sweep their wide stencil afterwards, each on its own lane.  Everything up to the
+// candidates that pass is FP32, widened by the slack that covers its rounding; about one
+// candidate in 500 passes and reads its two particles from the pool.  What bounds it is
+// instruction issue and the latency of the cell lookups.  Measured (B200): 16.8 M particles
+// 1.84 ms with FP64 home records in sorted columns -> 1.52, 1 M 0.105 -> 0.078.
 __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search(
-    const InstDev *__restrict__ insts, int64_t n, SearchArrays sa, PairRec *__restrict__ pairs,
-    unsigned long long *npairs, int64_t cap, Status *st) {
+    const InstDev *__restrict__ insts, const PoolView *__restrict__ pv, int64_t n, SearchArrays sa,
+    PairRec *__restrict__ pairs, unsigned long long *npairs, int64_t cap, Status *st) {
   // no halt test here: this kernel is what raises the flag, and a later block must not
   // skip its pairs because an earlier one overflowed (the count it leaves in
   // pairs_needed sizes the buffers).  In a step after a halted one the binning did not
-  // run and every cell is empty (its counts were cleared), so the sweep finds nothing.
-  __shared__ HomeRec homes[kSearchThreads];
+  // run and every cell is empty (its counts are zero between binnings), so the sweep finds
+  // nothing.
   __shared__ HomeF homesf[kSearchThreads];
   __shared__ int32_t rstart[kSearchThreads][kMaxRanges];   // first sorted particle of a range
   __shared__ int32_t rcum[kSearchThreads][kMaxRanges];     // candidates of the home before it
   __shared__ int8_t rnum[kSearchThreads];
   constexpr unsigned kFull = 0xffffffffu;
+  const PoolView &P = *pv;
   const int t = threadIdx.x, lane = t & 31, wbase = t & ~31;
   const int64_t nact = sa.cell_start[sa.ncells];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -445,35 +450,29 @@ __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search
     int nr = 0;
     int32_t c = 0;
     bool large = false;
-    int cx = 0, cy = 0, cz = 0;
-    HomeRec hr;
     if (s < nact) {
-      hr.inst = sa.sinst[s];
-      const InstDev &I = insts[hr.inst];
-      hr.s = (int32_t)s;
-      hr.xp = sa.sx[s]; hr.yp = sa.sy[s]; hr.zp = sa.sz[s]; hr.rp = sa.sr[s];
-      hr.bp = sa.sbox[s];
-      hr.pslot = sa.sorted[s];
-      hr.idp = sa.sid[s];
-      homes[t] = hr;
-      homesf[t] = home_f(I, hr.xp, hr.yp, hr.zp, hr.rp);
-      const int nfx = I.nfx, nfy = I.nfy, nfz = I.nfz;
-      const bool perx = I.periodicity != 0;
-      // the binning pass's own cell of this particle (same inputs, same function)
-      cx = cell_coord(hr.xp, I.hfx, nfx); cy = cell_coord(hr.yp, I.hfy, nfy); cz = cell_coord(hr.zp, I.hfz, nfz);
-      const int64_t lc = ((int64_t)cz * nfy + cy) * nfx + cx;
-      large = sa.spk[s].w < 0.f;
+      const float4 p = sa.spk[s];
+      const int32_t pslot = sa.sorted[s], cell = sa.cell_of[pslot];
+      const InstDev &I = insts[P.inst[pslot]];
+      homesf[t] = home_f(I, p);
+      large = p.w < 0.f;
       if (!large) {
+        int cx, cy, cz;
+        cell_coords(I, cell, cx, cy, cz);
+        const int nfx = I.nfx, nfy = I.nfy, nfz = I.nfz;
+        const bool perx = I.periodicity != 0;
         // Small candidates have radius <= rcut, so only cells whose box comes within
         // R = rp + rcut of this particle can hold a partner: rows and end cells farther
         // away are skipped (distances to the neighbour boxes from the offsets inside the
-        // home cell, shortened by 1e-9 of the cell edge against rounding).
-        const double R = (hr.rp + I.rcut) * (1.0 + 1e-9), R2 = R * R;
-        const double fx = hr.xp - cx * I.hfx, fy = hr.yp - cy * I.hfy, fz = hr.zp - cz * I.hfz;
-        const double ex = 1e-9 * I.hfx, ey = 1e-9 * I.hfy, ez = 1e-9 * I.hfz;
-        const double dxl = fmax(fx - ex, 0.0), dxh = fmax(I.hfx - fx - ex, 0.0);
-        const double dyl = fmax(fy - ey, 0.0), dyh = fmax(I.hfy - fy - ey, 0.0);
-        const double dzh = fmax(I.hfz - fz - ez, 0.0);
+        // home cell, shortened by the slack).
+        const float e = I.slack, rp = p.w * (1.0f + 1e-6f);
+        const float hx = (float)I.hfx, hy = (float)I.hfy, hz = (float)I.hfz;
+        const float R = rp + (float)I.rcut * (1.0f + 1e-6f), R2 = R * R;
+        const float fx = p.x - cx * hx, fy = p.y - cy * hy, fz = p.z - cz * hz;
+        const float dxl = fmaxf(fx - e, 0.f), dxh = fmaxf(hx - fx - e, 0.f);
+        const float dyl = fmaxf(fy - e, 0.f), dyh = fmaxf(hy - fy - e, 0.f);
+        const float dzh = fmaxf(hz - fz - e, 0.f);
+        const bool left_ok = (cx - 1 >= 0 || perx), right_ok = (cx + 1 < nfx || perx);
         auto add = [&](int32_t a0, int32_t a1) {
           if (a1 > a0) {
             rstart[t][nr] = a0;
@@ -483,42 +482,44 @@ __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search
           }
         };
         for (int r = 0; r < 5; ++r) {
-          int ry = cy, rz = cz, lo = cx - 1, hi = cx + 1;
-          double dyz2 = 0.0;
-          if (r == 0) {
-            lo = hi = cx + 1;                    // the rest of the home cell is taken below
-          } else if (r == 1) {
+          int ry = cy, rz = cz;
+          float dyz2 = 0.f;
+          if (r == 1) {
             ry = wrap_cell(cy + 1, nfy);
             dyz2 = dyh * dyh;
-          } else {
+          } else if (r > 1) {
             rz = wrap_cell(cz + 1, nfz);
             ry = wrap_cell(cy + (r - 3), nfy);
-            const double dyb = (r == 2) ? dyl : (r == 4 ? dyh : 0.0);
+            const float dyb = (r == 2) ? dyl : (r == 4 ? dyh : 0.f);
             dyz2 = dyb * dyb + dzh * dzh;
           }
-          if (r > 0 && dyz2 > R2) continue;
-          const int64_t base = I.cell_begin + ((int64_t)rz * nfy + ry) * nfx;
-          // each end cell within reach of its own largest radius
-          auto reach2 = [&](int cell) {
-            const int w = cell < 0 ? cell + nfx : (cell >= nfx ? cell - nfx : cell);
-            const double rr_ = (hr.rp + (double)sa.cell_rmax[base + w]) * (1.0 + 1e-9);
-            return rr_ * rr_;
+          if (dyz2 > R2) continue;
+          const int32_t row = cell_row(I, ry, rz);
+          // each cell within reach of its own largest radius
+          auto reaches = [&](int32_t k, float d2) {
+            const float m = rp + sa.cell_rmax[k];
+            return d2 <= R2 && d2 <= m * m;
           };
-          const bool left_ok = (cx - 1 >= 0 || perx);
-          const bool right_ok = (cx + 1 < nfx || perx);
-          if (r > 0 && (!left_ok || dxl * dxl + dyz2 > R2 || dxl * dxl + dyz2 > reach2(cx - 1))) lo = cx;
-          const bool right = right_ok && dxh * dxh + dyz2 <= R2 && dxh * dxh + dyz2 <= reach2(cx + 1);
-          if (r > 0 && !right) hi = cx;
-          if (r > 0 && lo == cx && hi == cx && dyz2 > reach2(cx)) continue;
-          RowRanges rr = {0, 0, 0, 0};
-          if (r > 0 || right) rr = row_ranges(sa, base, nfx, lo, hi, perx);
-          if (r == 0) {
-            // home cell from s+1, contiguous with cell cx+1 when that is not wrapped
-            if (rr.a1 == 0 && rr.a0 == 0) rr.a1 = sa.cell_start[I.cell_begin + lc + 1];
-            rr.a0 = (int32_t)s + 1;
+          const int32_t cl = row + (cx > 0 ? cx - 1 : nfx - 1), cm = row + cx;
+          const int32_t cr = row + (cx + 1 < nfx ? cx + 1 : 0);
+          const bool use_l = r > 0 && left_ok && reaches(cl, dxl * dxl + dyz2);
+          const bool use_r = right_ok && reaches(cr, dxh * dxh + dyz2);
+          // the home cell from s+1 on; its neighbours' middle cell whenever an end is used
+          const bool use_m = r == 0 || use_l || use_r || reaches(cm, dyz2);
+          int32_t a0 = 0, a1 = 0;
+          if (use_m) {
+            a0 = r == 0 ? (int32_t)s + 1 : sa.cell_start[cm];
+            a1 = sa.cell_start[cm + 1];
           }
-          add(rr.a0, rr.a1);
-          add(rr.b0, rr.b1);
+          if (use_l) {
+            const int32_t b0 = sa.cell_start[cl];
+            if (cl + 1 == cm) a0 = b0; else add(b0, sa.cell_start[cl + 1]);
+          }
+          if (use_r) {
+            const int32_t b1 = sa.cell_start[cr + 1];
+            if (cr == cm + 1) a1 = b1; else add(sa.cell_start[cr], b1);
+          }
+          add(a0, a1);
         }
       }
     }
@@ -550,44 +551,38 @@ __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search
         const int no = rnum[to];
         while (j + 1 < no && rcum[to][j + 1] <= k) ++j;
         const int32_t q = rstart[to][j] + (k - rcum[to][j]);
-        if (near_float<false>(sa.spk[q], q, 0, homesf[to])) {
-          const HomeRec ho = homes[to];
-          const InstDev &I = insts[ho.inst];
-          SearchHome h;
-          h.s = ho.s; h.xp = ho.xp; h.yp = ho.yp; h.zp = ho.zp; h.rp = ho.rp;
-          h.bp = ho.bp; h.pslot = ho.pslot; h.idp = ho.idp;
-          h.perx = I.periodicity != 0;
-          search_candidate(I, sa, h, q, pairs, npairs, cap, st);
-        }
+        if (near_float<false>(sa.spk[q], q, 0, homesf[to]))
+          search_candidate(insts, P, sa, (int32_t)(s0 + o), q, pairs, npairs, cap, st);
       }
     }
     if (large) {
       // a particle above the cut: every cell within its radius plus the largest radius
-      const InstDev &I = insts[hr.inst];
+      const int32_t pslot = sa.sorted[s];
+      const InstDev &I = insts[P.inst[pslot]];
       const int nfx = I.nfx, nfy = I.nfy, nfz = I.nfz;
-      SearchHome h;
-      h.s = hr.s; h.xp = hr.xp; h.yp = hr.yp; h.zp = hr.zp; h.rp = hr.rp;
-      h.bp = hr.bp; h.pslot = hr.pslot; h.idp = hr.idp;
-      h.perx = I.periodicity != 0;
-      const HomeF hf = home_f(I, h.xp, h.yp, h.zp, h.rp);
-      const double reach = (h.rp + I.rmax) * (1.0 + 1.0e-6);
+      int cx, cy, cz;
+      cell_coords(I, sa.cell_of[pslot], cx, cy, cz);
+      const HomeF hf = homesf[t];
+      const bool perx = I.periodicity != 0;
+      const double reach = (fmax(P.pc[0][pslot], P.pc[1][pslot]) + I.rmax) * (1.0 + 1.0e-6);
       const int rx = (int)ceil(reach / I.hfx), ry = (int)ceil(reach / I.hfy), rz = (int)ceil(reach / I.hfz);
-      const bool ally = 2 * ry + 1 >= nfy, allz = 2 * rz + 1 >= nfz;
+      const bool ally = 2 * ry + 1 >= nfy, allz = 2 * rz + 1 >= nfz, allx = 2 * rx + 1 >= nfx;
       const int y0 = ally ? 0 : cy - ry, y1 = ally ? nfy - 1 : cy + ry;
       const int z0 = allz ? 0 : cz - rz, z1 = allz ? nfz - 1 : cz + rz;
-      const int lo = (2 * rx + 1 >= nfx) ? 0 : cx - rx, hi = (2 * rx + 1 >= nfx) ? nfx - 1 : cx + rx;
+      int lo = allx ? 0 : cx - rx, hi = allx ? nfx - 1 : cx + rx;
+      if (!perx) { lo = max(lo, 0); hi = min(hi, nfx - 1); }
       for (int zz = z0; zz <= z1; ++zz) {
         const int wz = wrap_cell(zz, nfz);
         for (int yy = y0; yy <= y1; ++yy) {
-          const int wy = wrap_cell(yy, nfy);
-          const int64_t base = I.cell_begin + ((int64_t)wz * nfy + wy) * nfx;
-          const RowRanges rr = row_ranges(sa, base, nfx, lo, hi, h.perx || (2 * rx + 1 >= nfx));
-          for (int32_t qs = rr.a0; qs < rr.a1; ++qs)
-            if (qs != s && near_float<true>(sa.spk[qs], qs, h.s, hf))
-              search_candidate(I, sa, h, qs, pairs, npairs, cap, st);
-          for (int32_t qs = rr.b0; qs < rr.b1; ++qs)
-            if (qs != s && near_float<true>(sa.spk[qs], qs, h.s, hf))
-              search_candidate(I, sa, h, qs, pairs, npairs, cap, st);
+          const int32_t row = cell_row(I, wrap_cell(yy, nfy), wz);
+          for (int x = lo; x <= hi;) {
+            const int w = wrap_cell(x, nfx), len = min(nfx - w, hi - x + 1);   // up to the row's end
+            const int32_t q1 = sa.cell_start[row + w + len];
+            for (int32_t qs = sa.cell_start[row + w]; qs < q1; ++qs)
+              if (qs != s && near_float<true>(sa.spk[qs], qs, (int32_t)s, hf))
+                search_candidate(insts, P, sa, (int32_t)s, qs, pairs, npairs, cap, st);
+            x += len;
+          }
         }
       }
     }
@@ -595,9 +590,9 @@ __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search
   }
 }
 
-void launch_search(const InstDev *insts, int64_t n, SearchArrays sa, PairRec *pairs, unsigned long long *npairs,
+void launch_search(const InstDev *insts, const PoolView *pv, int64_t n, SearchArrays sa, PairRec *pairs, unsigned long long *npairs,
                    int64_t cap_pairs, Status *st, int grid, cudaStream_t s) {
-  k_search<<<grid, 256, 0, s>>>(insts, n, sa, pairs, npairs, cap_pairs, st);
+  k_search<<<grid, 256, 0, s>>>(insts, pv, n, sa, pairs, npairs, cap_pairs, st);
 }
 
 // ---------------------------------------------------------------------------

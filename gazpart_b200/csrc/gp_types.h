@@ -25,8 +25,10 @@ struct InstDev {
   // search grid (cell edge >= 2 * largest bounding radius)
   int32_t nfx, nfy, nfz, pad1;
   double hfx, hfy, hfz, rmax;
+  double ihfx, ihfy, ihfz;     // 1 / cell edge
   double rcut;                // particles with a larger bounding radius search a wider stencil
   int64_t cell_begin;         // first cell of this instance in the global cell arrays
+  float slack, pad2;          // bounds the rounding of FP32 positions and their differences
 };
 
 // Double-buffered structure-of-arrays particle pool.  Column j of buffer b is
@@ -109,19 +111,13 @@ struct ContactStatRec {
 
 // Binned particles of the collision search grid (see gp_search.cu).
 struct SearchArrays {
-  int32_t *cell_count;   // per search cell (+1 zero sentinel)
+  int32_t *cell_count;   // per search cell, zero between binnings
   int32_t *cell_start;   // exclusive scan, ncells+1
-  int32_t *cell_fill;
-  float *cell_rmax;       // per search cell: largest bounding radius of its small particles
+  float *cell_rmax;      // per search cell: largest bounding radius of its small particles
   int32_t *cell_of;      // per pool slot
   int32_t *sorted;       // pool slot of each sorted position
-  double *sx, *sy, *sz, *sr;
-  float4 *spk;           // (x, y, z, r) in float for the conservative first test
-  double *sex, *sey, *sez;   // symmetry axis in the lab frame (first column of R(q))
-  double *sa2, *sb2;         // squared semi-axes along / across the axis
-  long long *sbox;       // packed box coords (I0-1) | (J0-1)<<21 | (K0-1)<<42, -1 if outside
-  int32_t *sinst;
-  int32_t *sid;          // index of the particle within its instance
+  float4 *spk;           // per sorted position: (x, y, z, bounding radius) in float for the
+                         // conservative first test; the radius negated above the cut
   uint32_t *mark;        // per pool slot, non-null when the search flags pair members (speculative integrate)
   int64_t ncells;
 };
