@@ -38,28 +38,179 @@ void launch_integrate_fix_fp64(const InstDev *insts, PoolView *pv, PoolView *pv_
 }
 
 // INTERP_LAG3 (interp_lag3.f90:11-298) for one component at arbitrary points.
-__global__ void k_interp(const InstDev *__restrict__ inst, int comp, int64_t n, const double *__restrict__ x,
-                         const double *__restrict__ y, const double *__restrict__ z, double *__restrict__ out,
-                         Status *st) {
-  const InstDev I = *inst;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
-    Stencil s;
-    if (!stencil(I, x[p], y[p], z[p], s)) {
-      out[p] = CUDART_NAN;
-      set_error(st, GP_EOUT_OF_GRID, p);
-      continue;
+//
+// The points come in any order, and each touches 64 sectors of the field, so on a field
+// beyond the L2 nearly every sector comes from DRAM, half used or less.  Such calls
+// (sort_points in gp_api.cu has the rule and its measurements) first sort the points by the
+// mesh cell they lie in (a counting sort of their indices: row of cells, then runs of
+// 2^shift cells in x), so that the sectors are fetched about once; what bounds the sorted
+// call is the 64 sectors a point from the L2 (2 KB, 6 TB/s at 256^3 and 2 M points).
+//
+// One component of one stencil, single lane, in the reference's order (FP64) or as
+// gather6_fp32 sums it (mixed field).
+template <bool kMixed>
+__device__ __forceinline__ double interp_lane(const InstDev &I, const Stencil &s, int comp) {
+  if (kMixed) {
+    const float *__restrict__ F = static_cast<const float *>(I.field) + comp;
+    float fx[4], fy[4], fz[4];
+    lag3_wf((float)s.alfa, fx);
+    lag3_wf((float)s.beta, fy);
+    lag3_wf((float)s.gama, fz);
+    float sum = 0.f, cmp = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        const float wyz = fz[kk] * fy[jj];
+#pragma unroll
+        for (int ii = 0; ii < 4; ++ii) {
+          const float w = wyz * fx[ii];
+          const float v = __ldg(F + field_point(I, s.ix[ii], s.j0 - 1 + jj, s.k0 - 1 + kk) * kFieldStride);
+          const float y = __fmaf_rn(w, v, -cmp);
+          const float t = __fadd_rn(sum, y);
+          cmp = __fsub_rn(__fsub_rn(t, sum), y);
+          sum = t;
+        }
+      }
+    return (double)sum - (double)cmp;
+  }
+  const double *__restrict__ F = static_cast<const double *>(I.field) + comp;
+  double fx[4], fy[4], fz[4];
+  lag3_w(s.alfa, fx);
+  lag3_w(s.beta, fy);
+  lag3_w(s.gama, fz);
+  double zs = 0.0;
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk) {
+    double ys = 0.0;
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      double v[4];
+#pragma unroll
+      for (int ii = 0; ii < 4; ++ii)
+        v[ii] = __ldg(F + field_point(I, s.ix[ii], s.j0 - 1 + jj, s.k0 - 1 + kk) * kFieldStride);
+      const double xs = fx[0] * v[0] + fx[1] * v[1] + fx[2] * v[2] + fx[3] * v[3];
+      ys = (jj == 0) ? fy[0] * xs : ys + fy[jj] * xs;
     }
-    double g[6];
-    if (I.fprec == GP_PREC_MIXED) gather6_fp32(I, s, g); else gather6_fp64(I, s, g);
-    out[p] = g[comp];
+    zs = (kk == 0) ? fz[0] * ys : zs + fz[kk] * ys;
+  }
+  return zs;
+}
+
+// A warp's 32 points, FP64 field: sixteen lanes take one point, lane t the stencil row of
+// plane t >> 2 and line t & 3; the row sums are then added line by line and plane by plane
+// in the reference's order.  ok: this lane's point has a stencil contiguous in x.
+__device__ __forceinline__ double interp_warp(const InstDev &I, bool ok, int64_t b, const Stencil &s, int comp) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31, base = lane & 16, kk = (lane >> 2) & 3, c = lane & 3;
+  const double w0 = c == 0 ? -1. / 6. : (c == 1 ? 1. / 2. : (c == 2 ? -1. / 2. : 1. / 6.));
+  const int64_t sy = I.nx + 3, sz = (int64_t)(I.ny + 4) * sy;
+  const double *__restrict__ F = static_cast<const double *>(I.field) + comp + (kk * sz + c * sy) * kFieldStride;
+  double mine = 0.0;
+#pragma unroll 1
+  for (int g = 0; g < 16; ++g) {
+    const int o = 2 * g + (lane >> 4);
+    const bool oo = __shfl_sync(kFull, (int)ok, o) != 0;
+    const long long bo = __shfl_sync(kFull, (long long)b, o);
+    const double ax = __shfl_sync(kFull, s.alfa, o), ay = __shfl_sync(kFull, s.beta, o);
+    const double az = __shfl_sync(kFull, s.gama, o);
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    if (oo) {
+#pragma unroll
+      for (int ii = 0; ii < 4; ++ii) v[ii] = __ldg(F + (bo + ii) * kFieldStride);
+    }
+    // lane t forms weight t & 3 of axis t >> 2 (lag3_w's factors, in its order)
+    const double a = kk == 0 ? ax : (kk == 1 ? ay : az);
+    const double w = w0 * (a - (c == 3 ? 1. : 2.)) * (c < 2 ? a - 1. : a) * (c == 0 ? a : a + 1.);
+    double fx[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) fx[i] = __shfl_sync(kFull, w, base + i);
+    const double fy = __shfl_sync(kFull, w, base + 4 + c), fz = __shfl_sync(kFull, w, base + 8 + kk);
+    const double p = fy * (fx[0] * v[0] + fx[1] * v[1] + fx[2] * v[2] + fx[3] * v[3]);
+    double y = p;
+#pragma unroll
+    for (int d = 1; d < 4; ++d) y = y + __shfl_down_sync(kFull, p, d);   // right in the lanes with c = 0
+    const double q = fz * y;
+    double z = q;
+#pragma unroll
+    for (int d = 4; d < 16; d += 4) z = z + __shfl_down_sync(kFull, q, d);   // right in lanes 0 and 16
+    z = __shfl_sync(kFull, z, (lane & 1) << 4);
+    if ((lane >> 1) == g) mine = z;
+  }
+  return mine;
+}
+
+template <bool kMixed>
+__global__ void __launch_bounds__(256) k_interp(const InstDev *__restrict__ inst, int comp, int64_t n,
+                                                const int32_t *__restrict__ order, const double *__restrict__ x,
+                                                const double *__restrict__ y, const double *__restrict__ z,
+                                                double *__restrict__ out, Status *st) {
+  const InstDev I = *inst;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, nround = (n + 31) / 32 * 32;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nround; e += stride) {
+    Stencil s = {};
+    int64_t p = -1;
+    bool in = false;
+    if (e < n) {
+      p = order ? order[e] : e;
+      in = stencil(I, x[p], y[p], z[p], s);
+      if (!in) {
+        out[p] = CUDART_NAN;
+        set_error(st, GP_EOUT_OF_GRID, p);
+      }
+    }
+    if (kMixed) {
+      if (in) out[p] = interp_lane<true>(I, s, comp);
+    } else {
+      const bool row = in && s.contiguous;
+      const double v = interp_warp(I, row, row ? field_point(I, s.ix[0], s.j0 - 1, s.k0 - 1) : 0, s, comp);
+      if (row) out[p] = v;
+      else if (in) out[p] = interp_lane<false>(I, s, comp);
+    }
   }
 }
 
-void launch_interp(const InstDev *inst, int comp, int64_t n, const double *x, const double *y, const double *z,
-                   double *out, Status *st, cudaStream_t s) {
+// Bin of a point: its row of mesh cells and its run of 2^shift cells in it; points outside
+// the stencil's range go to bin 0.
+__global__ void k_point_bins(const InstDev *__restrict__ inst, int64_t n, int shift, const double *__restrict__ x,
+                             const double *__restrict__ y, const double *__restrict__ z, uint32_t *__restrict__ key,
+                             int32_t *__restrict__ count) {
+  const InstDev I = *inst;
+  const double ix = 1.0 / I.dx, iy = 1.0 / I.dy, iz = 1.0 / I.dz;
+  const int runs = (I.nx >> shift) + 1;
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
+    const double fx = x[p] * ix, fy = y[p] * iy, fz = z[p] * iz;
+    uint32_t k = 0u;
+    if (fx >= 0.0 && fx < (double)I.nx && fy >= 0.0 && fy < (double)I.ny && fz >= 0.0 && fz < (double)I.nz)
+      k = ((uint32_t)(int)fz * (uint32_t)I.ny + (uint32_t)(int)fy) * (uint32_t)runs + ((uint32_t)(int)fx >> shift);
+    key[p] = k;
+    atomicAdd(&count[k], 1);
+  }
+}
+
+__global__ void k_point_order(int64_t n, const uint32_t *__restrict__ key, const int32_t *__restrict__ start,
+                              int32_t *__restrict__ count, int32_t *__restrict__ order) {
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t k = key[p];
+    order[start[k] + atomicSub(&count[k], 1) - 1] = (int32_t)p;
+  }
+}
+
+static int point_grid(int64_t n) { return (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16); }
+
+void launch_point_order(const InstDev *inst, int64_t n, int shift, int64_t bins, const double *x, const double *y,
+                        const double *z, uint32_t *key, int32_t *count, int32_t *start, int32_t *scan_tmp,
+                        int32_t *order, cudaStream_t s) {
+  k_point_bins<<<point_grid(n), 256, 0, s>>>(inst, n, shift, x, y, z, key, count);
+  launch_scan(count, start, bins, scan_tmp, nullptr, s);
+  k_point_order<<<point_grid(n), 256, 0, s>>>(n, key, start, count, order);
+}
+
+void launch_interp(const InstDev *inst, bool mixed, int comp, int64_t n, const int32_t *order, const double *x,
+                   const double *y, const double *z, double *out, Status *st, cudaStream_t s) {
   if (n <= 0) return;
-  const int grid = (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
-  k_interp<<<grid, 256, 0, s>>>(inst, comp, n, x, y, z, out, st);
+  if (mixed) k_interp<true><<<point_grid(n), 256, 0, s>>>(inst, comp, n, order, x, y, z, out, st);
+  else k_interp<false><<<point_grid(n), 256, 0, s>>>(inst, comp, n, order, x, y, z, out, st);
 }
 
 // FROZEN_INTERP_LAG3 (frozen_interp_lag3.f90:11-274): plain (NX,NY,NZ) array, mirror

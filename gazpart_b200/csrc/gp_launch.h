@@ -21,8 +21,15 @@ void launch_integrate_fp64(const InstDev *insts, PoolView *pv, PoolView *pv_alt,
 void launch_integrate_fix_fp64(const InstDev *insts, PoolView *pv, PoolView *pv_alt, const PairRec *pairs,
                              const unsigned long long *npairs, int64_t cap_pairs, double *const *fluid,
                              uint32_t *mark, Status *st, int grid, cudaStream_t s);
-void launch_interp(const InstDev *inst, int comp, int64_t n, const double *x, const double *y, const double *z,
-                   double *out, Status *st, cudaStream_t s);
+// order (or null): the indices of the points in the order to take them, as
+// launch_point_order leaves them (bins: rows of mesh cells cut into runs of 2^shift cells,
+// ny * nz * ((nx >> shift) + 1) of them; count: bins + 1 zeros;
+// start: bins + 1; scan_tmp: scan_block_sums_size(bins); key, order: n).
+void launch_interp(const InstDev *inst, bool mixed, int comp, int64_t n, const int32_t *order, const double *x,
+                   const double *y, const double *z, double *out, Status *st, cudaStream_t s);
+void launch_point_order(const InstDev *inst, int64_t n, int shift, int64_t bins, const double *x, const double *y,
+                        const double *z, uint32_t *key, int32_t *count, int32_t *start, int32_t *scan_tmp,
+                        int32_t *order, cudaStream_t s);
 void launch_frozen_interp(const double *xain, const double *yain, const double *zain, int nx, int ny, int nz,
                           const double *uain, int64_t n, const double *x, const double *y, const double *z,
                           double *out, Status *st, cudaStream_t s);
