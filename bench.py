@@ -254,9 +254,9 @@ def cpu_sample(w, scale: int, max_emaj: float):
 
 def phase_note(tune) -> str:
     """What the multi-step graph's phase times cover under the launch choices in use."""
-    if not tune or not tune.get("overlap_gather"):
+    if tune and not tune.get("overlap_gather"):
         return "one stream: each phase alone"
-    if tune.get("speculative_integrate"):
+    if tune and tune.get("speculative_integrate"):
         return ("gather and integrate of step s+1 (particles in none of step s's candidate pairs) overlap the "
                 "contact solves of step s on a second stream; 'integrate' times the pair members after the response")
     return "gather of step s+1 overlaps the contact solves of step s (two streams in the graph)"

@@ -157,9 +157,13 @@ struct gp_ctx {
   std::map<int, cudaGraphExec_t> graphs;
   // launch grids (blocks), GP_TUNE_* order; gp_autotune picks them on the live workload
   int tune[GP_NTUNE] = {148 * 8, 148 * 4, 148 * 4, 148 * 4};
-  // gather of step s+1 on the side stream, overlapping step s's contact solves; the
-  // autotuner keeps it only where it shortens the step
-  bool overlap = false;
+  // gather of step s+1 on the side stream, overlapping step s's contact solves (multi-step
+  // graphs).  The solves end one by one and leave SMs idle, so it pays at every size: ms a
+  // step of five-step graphs without / with it (B200), FP64 10,000 particles 0.173 / 0.160,
+  // 20,000 packed 0.389 / 0.372, 1 M 1.158 / 1.012, 4 M 3.98 / 3.74; mixed 100,000 0.265 /
+  // 0.245, 1 M 0.850 / 0.750, 16.8 M 8.81 / 8.54, 24 classes of 2 M in all 1.366 / 1.269.
+  // The autotuner times both, and the speculative integrate too.
+  bool overlap = true;
   // with the overlap, step s+1's integrate also runs on the side stream, speculatively,
   // for the particles in no candidate pair of step s; the rest follow after the response
   // (d_mark: per pool slot, zero between steps; allocated while spec is on)
