@@ -7,8 +7,8 @@
 // that independent ones do not overlap either (eight independent divisions: 8 x 113
 // cycles).  A step has about 45 of them.  Here they are branch-free: a quotient is a
 // hardware seed, a cubic Newton step and one correction with an exact remainder, so that
-// independent ones fill each other's latency and several quotients by one divisor share
-// its reciprocal.  The step holds its state in registers (nothing is passed by address),
+// independent ones fill each other's latency, several quotients by one divisor share its
+// reciprocal, and a root brings the reciprocal of itself along.  The step holds its state in registers (nothing is passed by address),
 // takes the pivot column's norm once and leaves out what lm_step forms and never reads.
 // Operands outside the range in which the short forms are sound raise a flag, and a
 // flagged step is run by lm_step: 49 of 2.87 M steps of 150,000 pairs shaped like those
@@ -16,8 +16,8 @@
 //
 // Measured (B200, such pairs; kernel time, results identical bit for bit):
 //   one solve         6.2 us a step -> 1.9
-//   2,000 solves      0.81 ms -> 0.23 (the longest takes 128 steps)
-//   150,000 solves    2.45 ms -> 1.01
+//   2,000 solves      0.81 ms -> 0.22 (the longest takes 128 steps)
+//   150,000 solves    2.45 ms -> 0.90
 #pragma once
 #include "gp_lm.cuh"
 
@@ -79,36 +79,34 @@ GP_LF double lf_div(double a, double b, LfGuard& g) {
   g.in(a);
   return lf_quot(a, r);
 }
-// 1 / b and 0.5 / b: the numerators need no check
-GP_LF double lf_inv(double b, LfGuard& g) { return lf_quot(1.0, lf_rcp(b, g)); }
-
-// sqrt(a): hardware seed of 1/sqrt, a cubic Newton step for the root, one correction with
-// the exact remainder a - s^2 (as above; same condition).  The caller checks a.
-GP_LF double lf_sqrt_checked(double a) {
+// sqrt(a) and the reciprocal of that root: hardware seed of 1/sqrt, a cubic Newton step for
+// both, one correction of the root with the exact remainder a - s^2 (as above; same
+// condition).  1/sqrt(a) is within 1.5 ulp of 1/s, so a quotient by the root needs no
+// reciprocal of its own.  The caller checks a.
+GP_LF LfRcp lf_root(double a) {
   double y0;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
   const double t = __dmul_rn(a, y0);
   const double e = __fma_rn(-t, y0, 1.0);
   const double pe = __dmul_rn(e, __fma_rn(0.375, e, 0.5));
-  const double s = __fma_rn(t, pe, t);
-  const double h = __dmul_rn(0.5, __fma_rn(y0, pe, y0));
-  return __fma_rn(__fma_rn(-s, s, a), h, s);
+  const double s = __fma_rn(t, pe, t), y = __fma_rn(y0, pe, y0);
+  return {__fma_rn(__fma_rn(-s, s, a), __dmul_rn(0.5, y), s), y};
 }
 GP_LF double lf_sqrt(double a, LfGuard& g) {
   g.in(a);
-  return lf_sqrt_checked(a);
+  return lf_root(a).b;
 }
 
-// MINPACK's norm (lm_enorm) where it is sqrt of the sum of squares.
-GP_LF double lf_norm2(double x, double y, LfGuard& g) {
+// MINPACK's norm (lm_enorm) where it is sqrt of the sum of squares, with its reciprocal.
+GP_LF LfRcp lf_norm2(double x, double y, LfGuard& g) {
   const double s = x * x + y * y;
   g.norm(s, min(g.high(x), g.high(y)));
-  return lf_sqrt_checked(s);
+  return lf_root(s);
 }
-GP_LF double lf_norm3(double x, double y, double z, LfGuard& g) {
+GP_LF LfRcp lf_norm3(double x, double y, double z, LfGuard& g) {
   const double s = x * x + y * y + z * z;
   g.norm(s, min(g.high(x), min(g.high(y), g.high(z))));
-  return lf_sqrt_checked(s);
+  return lf_root(s);
 }
 
 // ct_sincos without its range branch (the caller's guard covers it) and its switch.
@@ -136,10 +134,15 @@ GP_LF void lf_support(const Prob& P, double x0, double x1, SupportEval& E, LfGua
   double t1[3], t2[3];
   prob_matvec<0>(P, c1, t1);
   prob_matvec<1>(P, c2, t2);
-  E.l1 = lf_sqrt(0.25 * (c1[0] * t1[0] + c1[1] * t1[1] + c1[2] * t1[2]), g);
-  E.l2 = lf_sqrt(0.25 * (c2[0] * t2[0] + c2[1] * t2[1] + c2[2] * t2[2]), g);
-  E.f1 = lf_inv(2.0 * E.l1, g);
-  E.f2 = lf_inv(2.0 * E.l2, g);
+  const double q1 = 0.25 * (c1[0] * t1[0] + c1[1] * t1[1] + c1[2] * t1[2]);
+  const double q2 = 0.25 * (c2[0] * t2[0] + c2[1] * t2[1] + c2[2] * t2[2]);
+  g.in(q1);
+  g.in(q2);
+  const LfRcp l1 = lf_root(q1), l2 = lf_root(q2);
+  E.l1 = l1.b;
+  E.l2 = l2.b;
+  E.f1 = lf_quot(1.0, {2.0 * l1.b, 0.5 * l1.y});
+  E.f2 = lf_quot(1.0, {2.0 * l2.b, 0.5 * l2.y});
 #pragma unroll
   for (int i = 0; i < 3; ++i)
     E.depth[i] = (E.f1 * t1[i] + P.template b<0>(i)) - (E.f2 * t2[i] + P.template b<1>(i));
@@ -153,7 +156,10 @@ GP_LF void lf_grad(const Prob& P, const double c[3], double l, double s, const d
 #pragma unroll
   for (int j = 0; j < 3; ++j)
     row[j] = c[0] * P.template e<W>(3 * j) + c[1] * P.template e<W>(1 + 3 * j) + c[2] * P.template e<W>(2 + 3 * j);
-  const double t = lf_inv(8.0 * (l * l * l), g);
+  // 1 / (8 l^3) from s = 1 / (2 l): s^3 is within 3 ulp of it
+  const double l3 = 8.0 * (l * l * l);
+  g.in(l3);
+  const double t = lf_quot(1.0, {l3, s * s * s});
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     double co[3];
@@ -172,7 +178,7 @@ GP_LF void lf_grad(const Prob& P, const double c[3], double l, double s, const d
 GP_LF void lf_givens(double r, double sd, double& cs, double& sn, LfGuard& g) {
   const bool big = fabs(r) >= fabs(sd);
   const double t = lf_div(big ? sd : r, big ? r : sd, g);
-  const double u = lf_quot(0.5, lf_rcp(lf_sqrt_checked(0.25 + 0.25 * (t * t)), g));
+  const double u = lf_quot(0.5, lf_root(0.25 + 0.25 * (t * t)));
   const double v = u * t;
   cs = big ? u : v;
   sn = big ? v : u;
@@ -204,7 +210,8 @@ GP_LF int lm_step_fast(const Prob& P, LmState& S, double tol, bool& ok) {
       }
     }
     // lm_qrfac: the pivot column's norm is the one already taken
-    const double ac0 = lf_norm3(a[0], a[1], a[2], g), ac1 = lf_norm3(a[3], a[4], a[5], g);
+    const LfRcp c0 = lf_norm3(a[0], a[1], a[2], g), c1 = lf_norm3(a[3], a[4], a[5], g);
+    const double ac0 = c0.b, ac1 = c1.b;
     const bool sw = ac1 > ac0;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -212,9 +219,9 @@ GP_LF int lm_step_fast(const Prob& P, LmState& S, double tol, bool& ok) {
       a[i] = sw ? a[i + 3] : t;
       a[i + 3] = sw ? t : a[i + 3];
     }
-    double n0 = sw ? ac1 : ac0;
-    if (a[0] < 0.0) n0 = -n0;
-    const LfRcp r0 = lf_rcp(n0, g);
+    LfRcp r0 = sw ? c1 : c0;
+    if (a[0] < 0.0) r0 = {-r0.b, -r0.y};
+    const double n0 = r0.b;
 #pragma unroll
     for (int i = 0; i < 3; ++i) a[i] = lf_div(a[i], r0, g);
     a[0] = a[0] + 1.0;
@@ -224,9 +231,9 @@ GP_LF int lm_step_fast(const Prob& P, LmState& S, double tol, bool& ok) {
 #pragma unroll
       for (int i = 0; i < 3; ++i) a[i + 3] = a[i + 3] - temp * a[i];
     }
-    double n1 = lf_norm2(a[4], a[5], g);
-    if (a[4] < 0.0) n1 = -n1;
-    const LfRcp r1 = lf_rcp(n1, g);
+    LfRcp r1 = lf_norm2(a[4], a[5], g);
+    if (a[4] < 0.0) r1 = {-r1.b, -r1.y};
+    const double n1 = r1.b;
     a[4] = lf_div(a[4], r1, g);
     a[5] = lf_div(a[5], r1, g);
     a[4] = a[4] + 1.0;
@@ -250,7 +257,7 @@ GP_LF int lm_step_fast(const Prob& P, LmState& S, double tol, bool& ok) {
     if (S.iter == 1) {
       d0 = ac0;
       d1 = ac1;
-      S.xnorm = lf_norm2(ac0 * S.x[0], ac1 * S.x[1], g);
+      S.xnorm = lf_norm2(ac0 * S.x[0], ac1 * S.x[1], g).b;
       S.delta = 100.0 * S.xnorm;
     }
     {
@@ -277,8 +284,8 @@ GP_LF int lm_step_fast(const Prob& P, LmState& S, double tol, bool& ok) {
     x1 = sel(sw, z1, z0);
     w0 = d0 * x0;
     w1 = d1 * x1;
-    double dxnorm = lf_norm2(w0, w1, g);
-    double fp = dxnorm - delta;
+    const LfRcp gauss = lf_norm2(w0, w1, g);
+    double fp = gauss.b - delta;
     if (fp <= 0.1 * delta) {
       par = 0.0;
     } else {
@@ -286,21 +293,20 @@ GP_LF int lm_step_fast(const Prob& P, LmState& S, double tol, bool& ok) {
       const LfRcp rdel = lf_rcp(delta, g);
       double parl, paru, gn;
       {
-        const LfRcp rn = lf_rcp(dxnorm, g);
-        double v0 = dp0 * lf_div(sel(sw, w0, w1), rn, g);
-        double v1 = dp1 * lf_div(sel(!sw, w0, w1), rn, g);
+        double v0 = dp0 * lf_div(sel(sw, w0, w1), gauss, g);
+        double v1 = dp1 * lf_div(sel(!sw, w0, w1), gauss, g);
         v0 = lf_div(v0 - 0.0, rr0, g);
         v1 = lf_div(v1 - (0.0 + R3 * v0), rr4, g);
-        const LfRcp rt = lf_rcp(lf_norm2(v0, v1, g), g);
+        const LfRcp rt = lf_norm2(v0, v1, g);
         parl = lf_div(lf_div(lf_div(fp, rdel, g), rt, g), rt, g);
         const double s0 = 0.0 + R0 * q0, s1 = (0.0 + R3 * q0) + R4 * q1;
-        gn = lf_norm2(lf_div(s0, dp0, g), lf_div(s1, dp1, g), g);
+        gn = lf_norm2(lf_div(s0, dp0, g), lf_div(s1, dp1, g), g).b;
         paru = lf_div(gn, rdel, g);
       }
       double p = par;
       p = (p > parl) ? p : parl;
       p = (p < paru) ? p : paru;
-      if (p == 0.0) p = lf_div(gn, dxnorm, g);
+      if (p == 0.0) p = lf_div(gn, gauss, g);
 #pragma unroll 1
       for (int iter = 1;; ++iter) {
         const double sp = lf_sqrt(p, g);
@@ -332,17 +338,16 @@ GP_LF int lm_step_fast(const Prob& P, LmState& S, double tol, bool& ok) {
         x1 = sel(sw, y1, y0);
         w0 = d0 * x0;
         w1 = d1 * x1;
-        dxnorm = lf_norm2(w0, w1, g);
+        const LfRcp rn = lf_norm2(w0, w1, g);
         const double told = fp;
-        fp = dxnorm - delta;
+        fp = rn.b - delta;
         if (fabs(fp) <= 0.1 * delta || (parl == 0.0 && fp <= told && told < 0.0) || iter == 10 || !g.ok()) break;
-        const LfRcp rn = lf_rcp(dxnorm, g);
         double v0 = dp0 * lf_div(sel(sw, w0, w1), rn, g);
         double v1 = dp1 * lf_div(sel(!sw, w0, w1), rn, g);
         v0 = lf_div(v0, rs0, g);
         v1 = v1 - r1 * v0;
         v1 = lf_div(v1, rs1, g);
-        const LfRcp rt = lf_rcp(lf_norm2(v0, v1, g), g);
+        const LfRcp rt = lf_norm2(v0, v1, g);
         const double parc = lf_div(lf_div(lf_div(fp, rdel, g), rt, g), rt, g);
         if (fp > 0.0) parl = (parl > p) ? parl : p;
         if (fp < 0.0) paru = (paru < p) ? paru : p;
@@ -355,16 +360,16 @@ GP_LF int lm_step_fast(const Prob& P, LmState& S, double tol, bool& ok) {
   // the trial point
   const double s0 = -x0, s1 = -x1;
   const double xt0 = S.x[0] + s0, xt1 = S.x[1] + s1;
-  const double pnorm = lf_norm2(d0 * s0, d1 * s1, g);
+  const double pnorm = lf_norm2(d0 * s0, d1 * s1, g).b;
   if (S.iter == 1) delta = (delta < pnorm) ? delta : pnorm;
   SupportEval E2;
   lf_support(P, xt0, xt1, E2, g);
-  const double fnorm1 = lf_norm3(E2.depth[0] * E2.depth[0], E2.depth[1] * E2.depth[1], E2.depth[2] * E2.depth[2], g);
+  const double fnorm1 = lf_norm3(E2.depth[0] * E2.depth[0], E2.depth[1] * E2.depth[1], E2.depth[2] * E2.depth[2], g).b;
   double actred = -1.0;
   if (0.1 * fnorm1 < S.fnorm) { const double r = lf_quot(fnorm1, rf); actred = 1.0 - r * r; }
   const double p0 = sel(sw, s0, s1), p1 = sel(!sw, s0, s1);
   const double v0 = (0.0 + R0 * p0) + R3 * p1, v1 = 0.0 + R4 * p1;
-  const double temp1 = lf_div(lf_norm2(v0, v1, g), rf, g);
+  const double temp1 = lf_div(lf_norm2(v0, v1, g).b, rf, g);
   double temp2 = 0.0;
   if (par != 0.0) temp2 = lf_div(lf_sqrt(par, g) * pnorm, rf, g);
   const double prered = temp1 * temp1 + (temp2 * temp2) * 2.0;
@@ -386,7 +391,7 @@ GP_LF int lm_step_fast(const Prob& P, LmState& S, double tol, bool& ok) {
   }
   const bool accept = ratio >= 1.0e-4;
   double xnorm = S.xnorm;
-  if (accept) xnorm = lf_norm2(d0 * xt0, d1 * xt1, g);
+  if (accept) xnorm = lf_norm2(d0 * xt0, d1 * xt1, g).b;
   ok = g.ok();
   if (!ok) return 0;
   ++S.nfev;
