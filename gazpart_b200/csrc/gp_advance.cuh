@@ -784,7 +784,7 @@ __device__ __forceinline__ void gather_warp_fp64(const InstDev* __restrict__ ins
 // Both gathers are warp-cooperative; stencils mirrored at a wall (not contiguous in x) are
 // left to their own lane.
 // Each warp takes the next `run` slots (a multiple of 4, at most 32; gather_run) from
-// *ticket (zero at launch), so the slots in
+// *ticket (zero at launch; finish_advance clears it), so the slots in
 // flight at any time are one contiguous run of the cell order whatever the grid: the
 // field rows that neighbouring stencils share stay in L2 between their uses, where a
 // grid-stride loop over many blocks spreads the resident warps over the pool.
@@ -930,6 +930,22 @@ __device__ __forceinline__ void integrate_slot(const InstDev* __restrict__ insts
   D->st[10][j] = O[0]; D->st[11][j] = O[1]; D->st[12][j] = O[2];
 }
 
+// The end of an advance, by the last block to get here (the views are read by nobody any
+// more): the destination buffer becomes the
+// current one and the gather's ticket goes back to zero (launches of their own otherwise).
+__device__ __forceinline__ void finish_advance(PoolView* a, PoolView* b, unsigned long long* done,
+                                               unsigned long long* ticket) {
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(done, 1ull) != (unsigned long long)gridDim.x - 1ull) return;
+  const PoolView t = *a;
+  *a = *b;
+  *b = t;
+  *done = 0ull;
+  *ticket = 0ull;
+}
+
 // The pass over the pool: particle perm[j] of the source buffer goes to slot j of the
 // destination.  With mark non-null (the speculative pass, run while the previous step's
 // contact solves and response are still going) a particle that the last search marked
@@ -941,12 +957,11 @@ __device__ __forceinline__ void integrate_slot(const InstDev* __restrict__ insts
 #define GP_INTEGRATE_MIN_BLOCKS 4
 #endif
 template <bool kMixed>
-__global__ void __launch_bounds__(128, GP_INTEGRATE_MIN_BLOCKS) k_integrate(const InstDev* __restrict__ insts,
-                                                                           const PoolView* __restrict__ src_pv,
-                                                                           const PoolView* __restrict__ dst_pv,
-                                                                           const int32_t* __restrict__ perm, int64_t n,
-                                                                           const double* const* __restrict__ fluid,
-                                                                           uint32_t* __restrict__ mark, Status* st) {
+__global__ void __launch_bounds__(128, GP_INTEGRATE_MIN_BLOCKS)
+    k_integrate(const InstDev* __restrict__ insts, const PoolView* __restrict__ src_pv,
+                const PoolView* __restrict__ dst_pv, const int32_t* __restrict__ perm, int64_t n,
+                const double* const* __restrict__ fluid, uint32_t* __restrict__ mark, PoolView* src, PoolView* dst,
+                unsigned long long* done, unsigned long long* ticket, Status* st) {
   if (step_halted(st)) return;
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = perm[j];
@@ -956,6 +971,7 @@ __global__ void __launch_bounds__(128, GP_INTEGRATE_MIN_BLOCKS) k_integrate(cons
     }
     integrate_slot<kMixed>(insts, src_pv, dst_pv, i, j, fluid, st);
   }
+  if (mark == nullptr) finish_advance(src, dst, done, ticket);
 }
 
 // The rest of a speculative pass, after the response: every particle of the stored
@@ -963,14 +979,12 @@ __global__ void __launch_bounds__(128, GP_INTEGRATE_MIN_BLOCKS) k_integrate(cons
 // first lane to clear its mark takes it), into the slot the speculative pass recorded.
 // The marks are all zero again afterwards.
 template <bool kMixed>
-__global__ void __launch_bounds__(128, GP_INTEGRATE_MIN_BLOCKS) k_integrate_fix(const InstDev* __restrict__ insts,
-                                                                               const PoolView* __restrict__ src_pv,
-                                                                               const PoolView* __restrict__ dst_pv,
-                                                                               const PairRec* __restrict__ pairs,
-                                                                               const unsigned long long* npairs,
-                                                                               int64_t cap,
-                                                                               const double* const* __restrict__ fluid,
-                                                                               uint32_t* __restrict__ mark, Status* st) {
+__global__ void __launch_bounds__(128, GP_INTEGRATE_MIN_BLOCKS)
+    k_integrate_fix(const InstDev* __restrict__ insts, const PoolView* __restrict__ src_pv,
+                    const PoolView* __restrict__ dst_pv, const PairRec* __restrict__ pairs,
+                    const unsigned long long* npairs, int64_t cap, const double* const* __restrict__ fluid,
+                    uint32_t* __restrict__ mark, PoolView* src, PoolView* dst, unsigned long long* done,
+                    unsigned long long* ticket, Status* st) {
   if (step_halted(st)) return;
   const int64_t np = (int64_t)min(*npairs, (unsigned long long)cap);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 2 * np; e += (int64_t)gridDim.x * blockDim.x) {
@@ -979,15 +993,7 @@ __global__ void __launch_bounds__(128, GP_INTEGRATE_MIN_BLOCKS) k_integrate_fix(
     const uint32_t v = atomicExch(&mark[i], 0u);
     if (v != 0u) integrate_slot<kMixed>(insts, src_pv, dst_pv, i, (int64_t)v - 1, fluid, st);
   }
-}
-
-// After an advance the destination buffer becomes the current one (not after an advance
-// that a halted step skipped).
-static __global__ void k_swap_pool(PoolView* a, PoolView* b, const Status* st) {
-  if (step_halted(st)) return;
-  const PoolView t = *a;
-  *a = *b;
-  *b = t;
+  finish_advance(src, dst, done, ticket);
 }
 
 }  // namespace gp

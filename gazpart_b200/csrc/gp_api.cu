@@ -135,15 +135,16 @@ struct gp_ctx {
   PoolView *d_pv_alt = nullptr;   // the other one
   // search
   SearchArrays sa{};
-  int32_t *d_scan_tmp = nullptr;
+  unsigned long long *d_scan_state = nullptr;   // scan_tiles(ncells_cap) words
   int64_t ncells = 0, ncells_cap = 0;
   PairRec *d_pairs = nullptr;
   int64_t cap_pairs = 0;
   CollRec *d_coll = nullptr;
   int64_t cap_coll = 0;
-  unsigned long long *d_counters = nullptr;   // [0] npairs [1] ncoll [2] nacc [4] contacts kept for the
-                                              // statistics [6] the gather's work ticket [7] collision steps
-                                              // in the statistics; from kPassCounters on, per contact pass,
+  unsigned long long *d_counters = nullptr;   // [0] npairs [1] ncoll [2] nacc [3] pairs to solve
+                                              // [4] contacts kept for the statistics [5] blocks of the
+                                              // integrate that are done [6] the gather's work ticket
+                                              // [7] collision steps in the statistics; from kPassCounters on, per contact pass,
                                               // its queue and the solves it hands over
   unsigned long long *d_best1 = nullptr, *d_best2 = nullptr;
   int8_t *d_matched = nullptr, *d_state = nullptr;
@@ -203,8 +204,8 @@ struct gp_ctx {
   // the mixed gather's staging: 0 stencil rows through L1, 1 each stencil box staged in
   // shared memory by the TMA (gp_gather_tma.cu), over gmap, the tensor map of gmap_field
   int gather_staging = 0;
-  // gp_interp_lag3's point order: one block of point_words words, for each call the bins'
-  // counters, their starts, the scan's sums, the points' bins and order
+  // gp_interp_lag3's point order: one block of point_words words, for each call the scan's
+  // tiles, the bins' counters and starts, the points' bins and order
   int32_t *d_points = nullptr;
   int64_t point_words = 0;
   CUtensorMap gmap{};
@@ -314,7 +315,7 @@ int class_props(gp_ctx *c, int ig, int idp, double pc[kNConst]) {
 
 void free_search(gp_ctx *c) {
   dfree(c->sa.cell_count); dfree(c->sa.cell_start); dfree(c->sa.cell_rmax);
-  dfree(c->d_scan_tmp);
+  dfree(c->d_scan_state);
   c->ncells_cap = 0;
 }
 
@@ -478,7 +479,7 @@ int alloc_cells(gp_ctx *c, int64_t ncells) {
     GP_TRY(dalloc(&c->sa.cell_start, ncells + 1));
     GP_TRY(dalloc(&c->sa.cell_rmax, ncells + 1));
     GP_CK(cudaMemsetAsync(c->sa.cell_count, 0, (ncells + 1) * sizeof(int32_t), c->stream));
-    GP_TRY(dalloc(&c->d_scan_tmp, (size_t)scan_block_sums_size(ncells)));
+    GP_TRY(dalloc(&c->d_scan_state, (size_t)scan_tiles(ncells)));
     c->ncells_cap = ncells;
   }
   c->ncells = ncells;
@@ -548,10 +549,10 @@ int enqueue_integrate(gp_ctx *c) {
   GP_TRY(mark(c, 2 * GP_PHASE_INTEGRATE, c->stream));
   if (c->prm.precision == GP_PREC_MIXED)
     launch_integrate_mixed(c->d_inst, c->d_pv, c->d_pv_alt, c->sa.sorted, c->n, c->d_fluid_cols, c->d_status,
-                           c->tune[GP_TUNE_INTEGRATE], c->stream);
+                           c->tune[GP_TUNE_INTEGRATE], c->d_counters + 5, c->d_counters + 6, c->stream);
   else
     launch_integrate_fp64(c->d_inst, c->d_pv, c->d_pv_alt, c->sa.sorted, c->n, c->d_fluid_cols, c->d_status,
-                          c->tune[GP_TUNE_INTEGRATE], c->stream);
+                           c->tune[GP_TUNE_INTEGRATE], c->d_counters + 5, c->d_counters + 6, c->stream);
   GP_CK(cudaGetLastError());
   c->n_slots = c->n;   // the pass writes the active particles, in cell order, to slots [0, n)
   c->fluid_ok = true;  // and the fluid it used, at the same slots
@@ -563,10 +564,10 @@ int enqueue_integrate(gp_ctx *c) {
 int enqueue_integrate_spec(gp_ctx *c, cudaStream_t s) {
   if (c->prm.precision == GP_PREC_MIXED)
     launch_integrate_mixed(c->d_inst, c->d_pv, c->d_pv_alt, c->sa.sorted, c->n, c->d_fluid_cols, c->d_status,
-                           c->tune[GP_TUNE_INTEGRATE], s, c->d_mark);
+                           c->tune[GP_TUNE_INTEGRATE], c->d_counters + 5, c->d_counters + 6, s, c->d_mark);
   else
     launch_integrate_fp64(c->d_inst, c->d_pv, c->d_pv_alt, c->sa.sorted, c->n, c->d_fluid_cols, c->d_status,
-                          c->tune[GP_TUNE_INTEGRATE], s, c->d_mark);
+                           c->tune[GP_TUNE_INTEGRATE], c->d_counters + 5, c->d_counters + 6, s, c->d_mark);
   GP_CK(cudaGetLastError());
   return GP_OK;
 }
@@ -577,10 +578,12 @@ int enqueue_integrate_fix(gp_ctx *c) {
   GP_TRY(mark(c, 2 * GP_PHASE_INTEGRATE, c->stream));
   if (c->prm.precision == GP_PREC_MIXED)
     launch_integrate_fix_mixed(c->d_inst, c->d_pv, c->d_pv_alt, c->d_pairs, c->d_counters + 0, c->cap_pairs,
-                               c->d_fluid_cols, c->d_mark, c->d_status, 148 * 4, c->stream);
+                               c->d_fluid_cols, c->d_mark, c->d_status, 148 * 4, c->d_counters + 5, c->d_counters + 6,
+                               c->stream);
   else
     launch_integrate_fix_fp64(c->d_inst, c->d_pv, c->d_pv_alt, c->d_pairs, c->d_counters + 0, c->cap_pairs,
-                              c->d_fluid_cols, c->d_mark, c->d_status, 148 * 4, c->stream);
+                              c->d_fluid_cols, c->d_mark, c->d_status, 148 * 4, c->d_counters + 5, c->d_counters + 6,
+                               c->stream);
   GP_CK(cudaGetLastError());
   c->n_slots = c->n;
   c->fluid_ok = true;
@@ -595,9 +598,12 @@ int enqueue_advance(gp_ctx *c) {
 // Binning of the search grid (also the cell order the next advance moves to).
 int enqueue_bin(gp_ctx *c) {
   SearchArrays sa = c->sa;
-  GP_CK(cudaMemsetAsync(c->d_counters, 0, 6 * sizeof(unsigned long long), c->stream));
-  launch_bin_count(c->d_inst, c->d_pv, c->n_slots, sa, c->d_status, c->tune[GP_TUNE_BIN], c->stream);
-  launch_scan(sa.cell_count, sa.cell_start, c->ncells, c->d_scan_tmp, sa.cell_rmax, c->stream);
+  // counters 0 to 5 and the contact passes'
+  const PhaseClear clear = {c->d_counters, 0x3Fu | (((1u << (2 * kMaxPasses)) - 1u) << kPassCounters),
+                            kPassCounters + 2 * kMaxPasses, c->d_qbins, 2 * kQueueBins, c->d_scan_state,
+                            scan_tiles(c->ncells)};
+  launch_bin_count(c->d_inst, c->d_pv, c->n_slots, sa, c->d_status, c->tune[GP_TUNE_BIN], clear, c->stream);
+  launch_scan(sa.cell_count, sa.cell_start, c->ncells, c->d_scan_state, sa.cell_rmax, c->d_status, c->stream);
   launch_bin_scatter(c->d_inst, c->d_pv, c->n_slots, sa, c->d_status, c->tune[GP_TUNE_BIN], c->stream);
   GP_CK(cudaGetLastError());
   return GP_OK;
@@ -620,10 +626,8 @@ int enqueue_bin_search(gp_ctx *c, bool flag = false) {
   // stream, so that the contact kernel is the first work ready after the fork and its
   // persistent grid takes the SMs before the gather's blocks do.
   if (qorder_ready(c)) {
-    GP_CK(cudaMemsetAsync(c->d_qbins, 0, 2 * kQueueBins * sizeof(uint32_t), c->stream));
     launch_queue_order(c->d_inst, c->d_pv, c->d_pairs, c->d_counters + 0, c->cap_pairs, c->d_evhist, c->n_slots,
-                       c->d_qkey, c->d_qbins, c->d_qorder, c->d_status, 148 * 4, c->stream);
-    GP_CK(cudaMemsetAsync(c->d_evhist, 0, (size_t)c->n_slots * sizeof(uint32_t), c->stream));
+                       c->d_qkey, c->d_qbins, c->d_qorder, c->d_counters + 3, c->d_status, 148 * 4, c->stream);
   }
   GP_CK(cudaGetLastError());
   return mark(c, 2 * GP_PHASE_SEARCH + 1, c->stream);
@@ -640,7 +644,6 @@ int enqueue_contact_response(gp_ctx *c) {
   for (int b = c->tail_budget; b > 0 && b < 300 && npass < kMaxPasses - 1; b *= 3) budget[npass++] = b;
   budget[npass++] = 0;
   unsigned long long *pc = c->d_counters + kPassCounters;
-  GP_CK(cudaMemsetAsync(pc, 0, 2 * kMaxPasses * sizeof(unsigned long long), c->stream));
   // the first pass takes the pairs in the order enqueue_bin_search formed
   const bool order = qorder_ready(c);
   const int64_t nhist = order ? c->n_slots : 0;
@@ -648,7 +651,7 @@ int enqueue_contact_response(gp_ctx *c) {
     const bool last = p == npass - 1;
     const TailRec *in = p > 0 ? c->d_tail[(p - 1) & 1] : nullptr;
     TailRec *out = last ? nullptr : c->d_tail[p & 1];
-    launch_contact(c->d_inst, c->d_pv, c->d_pairs, c->d_counters + 0, c->cap_pairs, in,
+    launch_contact(c->d_inst, c->d_pv, c->d_pairs, c->d_counters + (order && p == 0 ? 3 : 0), c->cap_pairs, in,
                    p > 0 ? pc + 2 * (p - 1) + 1 : nullptr, c->cap_tail, c->d_coll, c->d_counters + 1, c->cap_coll,
                    pc + 2 * p, cst, c->d_counters + 4, c->cap_cst, out, pc + 2 * p + 1, c->cap_tail, budget[p],
                    (order && p == 0) ? c->d_qorder : nullptr, order ? c->d_evhist : nullptr, nhist,
@@ -1706,12 +1709,12 @@ int gp_interp_lag3(gp_ctx *c, int32_t comp, int64_t nint, const double *xint, co
     int shift = 4;   // as many bins as points at most
     while (shift < 31 && (int64_t)I.ny * I.nz * ((I.nx >> shift) + 1) > nint && (I.nx >> shift) > 0) ++shift;
     const int64_t bins = (int64_t)I.ny * I.nz * ((I.nx >> shift) + 1);
-    const int64_t sums = scan_block_sums_size(bins);
-    if (bins < (int64_t(1) << 31) - 2 && point_workspace(c, 2 * (bins + 1) + sums + 2 * nint)) {
-      int32_t *count = c->d_points, *start = count + bins + 1, *tmp = start + bins + 1, *key = tmp + sums;
-      GP_CK(cudaMemsetAsync(count, 0, (bins + 1) * sizeof(int32_t), c->stream));
+    const int64_t tiles = 2 * scan_tiles(bins);   // words
+    if (bins < (int64_t(1) << 31) - 2 && point_workspace(c, tiles + 2 * (bins + 1) + 2 * nint)) {
+      int32_t *count = c->d_points + tiles, *start = count + bins + 1, *key = start + bins + 1;
+      GP_CK(cudaMemsetAsync(c->d_points, 0, (tiles + bins + 1) * sizeof(int32_t), c->stream));
       launch_point_order(c->d_inst, nint, shift, bins, dx, dy, dz, reinterpret_cast<uint32_t *>(key), count, start,
-                         tmp, key + nint, c->stream);
+                         reinterpret_cast<unsigned long long *>(c->d_points), key + nint, c->d_status, c->stream);
       order = key + nint;
     }
   }

@@ -9,7 +9,7 @@
 // 147,000 solves (512^3 / 16.8 M) four blocks at 128 registers took 0.98 ms against 1.01
 // in the solver alone, and up to 30% longer below 40,000 solves, so two blocks serve all
 // sizes.  Contact phase, before (eight blocks at 64 registers, the state in local memory)
-// and now: 0.26 -> 0.09 ms at 10,000 spheroids, 0.85 -> 0.23 at 1 M, 3.23 -> 1.16 at
+// and now: 0.26 -> 0.08 ms at 10,000 spheroids, 0.85 -> 0.20 at 1 M, 3.23 -> 0.93 at
 // 16.8 M.
 #include <math_constants.h>
 
@@ -18,24 +18,29 @@
 
 namespace gp {
 
-// Takes up pair e: false when its bodies are proven apart or there is nothing to solve.
-// Out of line, on the caller's copies, so that the solving loop keeps its problem and
-// state in registers; likewise the hand-over records of an earlier pass.
-static __device__ __noinline__ bool take_pair(const InstDev *__restrict__ insts, const PoolView *__restrict__ pv,
-                                              const PairRec *__restrict__ pairs, int64_t e, ContactProb &CP,
-                                              LmState &S) {
-  const PairRec pr = pairs[e];
-  PairBodies B;
-  pair_bodies(insts, *pv, pr.home, pr.near, B);
+// The pair's bodies are disjoint by the separation test: no contact, so no solve.
+__device__ __forceinline__ bool bodies_apart(const PairBodies &B) {
   const double vkx = B.c2[0] - B.c1[0], vky = B.c2[1] - B.c1[1], vkz = B.c2[2] - B.c1[2];
   const Quat &q1 = B.q1, &q2 = B.q2;
-  // symmetry axes (first columns of R(q)); disjoint bodies need no solve
+  // symmetry axes (first columns of R(q))
   const double e1[3] = {1.0 - 2.0 * (q1.c * q1.c + q1.d * q1.d), 2.0 * (q1.b * q1.c + q1.a * q1.d),
                         2.0 * (q1.b * q1.d - q1.a * q1.c)};
   const double e2[3] = {1.0 - 2.0 * (q2.c * q2.c + q2.d * q2.d), 2.0 * (q2.b * q2.c + q2.a * q2.d),
                         2.0 * (q2.b * q2.d - q2.a * q2.c)};
-  if (separated(vkx, vky, vkz, e1, B.a1 * B.a1, B.b1 * B.b1, e2, B.a2 * B.a2, B.b2 * B.b2)) return false;
-  return solve_start(B.a1, B.b1, B.a2, B.b2, B.c1, q1, B.c2, q2, CP, S);
+  return separated(vkx, vky, vkz, e1, B.a1 * B.a1, B.b1 * B.b1, e2, B.a2 * B.a2, B.b2 * B.b2);
+}
+
+// Takes up pair e: false when its bodies are proven apart (unless they were tested) or there
+// is nothing to solve.  Out of line, on the caller's copies, so that the solving loop keeps
+// its problem and state in registers; likewise the hand-over records of an earlier pass.
+static __device__ __noinline__ bool take_pair(const InstDev *__restrict__ insts, const PoolView *__restrict__ pv,
+                                              const PairRec *__restrict__ pairs, int64_t e, bool tested,
+                                              ContactProb &CP, LmState &S) {
+  const PairRec pr = pairs[e];
+  PairBodies B;
+  pair_bodies(insts, *pv, pr.home, pr.near, B);
+  if (!tested && bodies_apart(B)) return false;
+  return solve_start(B.a1, B.b1, B.a2, B.b2, B.c1, B.q1, B.c2, B.q2, CP, S);
 }
 
 // A solve handed over by an earlier pass: its pair and solver state, and the problem
@@ -64,35 +69,27 @@ static __device__ __noinline__ void resume_solve(const InstDev *__restrict__ ins
 // pair, never its result.
 //
 // hist[k] (k = the particle's instance begin + its id, below nhist) holds what the
-// particle's solves took in the last collision phase: 0 nothing (no candidate pair), 1
-// every pair proven apart before a solve, otherwise 1 + the largest evaluation count.  A
-// pair's prediction is the smaller of its two particles' values, and a pair with no
-// record at all (a new pair) is placed as a solve of typical length.
+// particle's solves took in the last collision phase: 0 nothing, otherwise 1 + the largest
+// evaluation count.  A pair's prediction is the smaller of its two particles' values, and a
+// pair with no record at all (a new pair) is placed as a solve of typical length.
+//
+// The pairs that the separation test proves apart (a third to a half) are left out here,
+// where every lane has a pair to test: in the contact kernel each of them took a lane of a
+// warp whose other lanes waited.  Bin kApart holds them.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kNewPairCost = 21;
+constexpr int kApart = kQueueBins - 1;
 
 __device__ __forceinline__ int64_t hist_index(const InstDev *__restrict__ insts, const PoolView &P, int slot) {
   return insts[P.inst[slot]].begin + P.id[slot];
 }
 
-// A pair proven apart without a solve, in the particles' record.  Out of line, so that
-// the refill path keeps its registers.
-static __device__ __noinline__ void record_apart(const InstDev *__restrict__ insts, const PoolView *__restrict__ pv,
-                                                 const PairRec *__restrict__ pairs, int64_t e, uint32_t *hist,
-                                                 int64_t nhist) {
-  const PoolView &P = *pv;
-  const PairRec pr = pairs[e];
-  const int64_t g1 = hist_index(insts, P, pr.home), g2 = hist_index(insts, P, pr.near);
-  if (g1 < nhist) atomicMax(&hist[g1], 1u);
-  if (g2 < nhist) atomicMax(&hist[g2], 1u);
-}
-
-__global__ void k_queue_count(const InstDev *__restrict__ insts, const PoolView *__restrict__ pv,
-                              const PairRec *__restrict__ pairs, const unsigned long long *__restrict__ npairs,
-                              int64_t cap_pairs, const uint32_t *__restrict__ hist, int64_t nhist,
-                              uint8_t *__restrict__ key, uint32_t *__restrict__ bins, const Status *st) {
+__global__ void __launch_bounds__(128) k_queue_count(
+    const InstDev *__restrict__ insts, const PoolView *__restrict__ pv, const PairRec *__restrict__ pairs,
+    const unsigned long long *__restrict__ npairs, int64_t cap_pairs, const uint32_t *__restrict__ hist,
+    int64_t nhist, uint8_t *__restrict__ key, uint32_t *__restrict__ bins, const Status *st) {
   if (step_halted(st)) return;
-  const PoolView P = *pv;
+  const PoolView &P = *pv;
   const int64_t np = (int64_t)min(*npairs, (unsigned long long)cap_pairs);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t nround = (np + stride - 1) / stride * stride;   // whole warps stay in the loop
@@ -100,10 +97,16 @@ __global__ void k_queue_count(const InstDev *__restrict__ insts, const PoolView 
     int k = -1;
     if (e < np) {
       const PairRec pr = pairs[e];
-      const int64_t g1 = hist_index(insts, P, pr.home), g2 = hist_index(insts, P, pr.near);
-      uint32_t p = (g1 < nhist && g2 < nhist) ? min(hist[g1], hist[g2]) : 0u;
-      if (p == 0u) p = kNewPairCost;
-      k = kQueueBins - 1 - (int)min(p, (uint32_t)(kQueueBins - 1));   // ascending bin = descending length
+      PairBodies B;
+      pair_bodies(insts, P, pr.home, pr.near, B);
+      if (bodies_apart(B)) {
+        k = kApart;
+      } else {
+        const int64_t g1 = hist_index(insts, P, pr.home), g2 = hist_index(insts, P, pr.near);
+        uint32_t p = (g1 < nhist && g2 < nhist) ? min(hist[g1], hist[g2]) : 0u;
+        if (p == 0u) p = kNewPairCost;
+        k = kApart - 1 - (int)min(p, (uint32_t)(kApart - 1));   // ascending bin = descending length
+      }
       key[e] = (uint8_t)k;
     }
     const unsigned peers = __match_any_sync(0xffffffffu, k);
@@ -113,11 +116,14 @@ __global__ void k_queue_count(const InstDev *__restrict__ insts, const PoolView 
 
 // order[start(bin) + fill] = e; every block forms the bins' starts itself (256 values).
 // bins[0, kQueueBins) are the counts, bins[kQueueBins, 2 kQueueBins) the fill counters.
+// The record has been read and is cleared for this phase's solves.
 __global__ void k_queue_scatter(const unsigned long long *__restrict__ npairs, int64_t cap_pairs,
                                 const uint8_t *__restrict__ key, uint32_t *__restrict__ bins,
-                                uint32_t *__restrict__ order, const Status *st) {
+                                uint32_t *__restrict__ order, unsigned long long *__restrict__ nsolve,
+                                uint32_t *__restrict__ hist, int64_t nhist, const Status *st) {
   if (step_halted(st)) return;
   __shared__ uint32_t start[kQueueBins];
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, gid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (threadIdx.x < 32) {
     uint32_t run = 0;
     for (int b0 = 0; b0 < kQueueBins; b0 += 32) {
@@ -131,14 +137,16 @@ __global__ void k_queue_scatter(const unsigned long long *__restrict__ npairs, i
       start[b0 + threadIdx.x] = run + x - v;
       run += __shfl_sync(0xffffffffu, x, 31);
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *nsolve = start[kApart];
   }
+  for (int64_t g = gid; g < nhist; g += stride) hist[g] = 0u;
   __syncthreads();
   const int64_t np = (int64_t)min(*npairs, (unsigned long long)cap_pairs);
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t nround = (np + stride - 1) / stride * stride;
   const int lane = threadIdx.x & 31;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nround; e += stride) {
-    const int k = (e < np) ? (int)key[e] : -1;
+  for (int64_t e = gid; e < nround; e += stride) {
+    int k = (e < np) ? (int)key[e] : -1;
+    if (k == kApart) k = -1;
     const unsigned peers = __match_any_sync(0xffffffffu, k);
     const int leader = __ffs(peers) - 1;
     uint32_t base = 0;
@@ -149,18 +157,19 @@ __global__ void k_queue_scatter(const unsigned long long *__restrict__ npairs, i
 }
 
 void launch_queue_order(const InstDev *insts, const PoolView *pv, const PairRec *pairs,
-                        const unsigned long long *npairs, int64_t cap_pairs, const uint32_t *hist, int64_t nhist,
-                        uint8_t *key, uint32_t *bins, uint32_t *order, const Status *st, int grid, cudaStream_t s) {
-  k_queue_count<<<grid, 256, 0, s>>>(insts, pv, pairs, npairs, cap_pairs, hist, nhist, key, bins, st);
-  k_queue_scatter<<<grid, 256, 0, s>>>(npairs, cap_pairs, key, bins, order, st);
+                        const unsigned long long *npairs, int64_t cap_pairs, uint32_t *hist, int64_t nhist,
+                        uint8_t *key, uint32_t *bins, uint32_t *order, unsigned long long *nsolve, const Status *st,
+                        int grid, cudaStream_t s) {
+  k_queue_count<<<2 * grid, 128, 0, s>>>(insts, pv, pairs, npairs, cap_pairs, hist, nhist, key, bins, st);
+  k_queue_scatter<<<grid, 256, 0, s>>>(npairs, cap_pairs, key, bins, order, nsolve, hist, nhist, st);
 }
 
 // collision_interaction.f90:216-348 for every candidate pair: minimum image, contact
 // (ellipsoid_contact_detection), contact-point velocities, NVREL.  Colliding pairs
 // (flag && NVREL < ZERO) are appended.  Persistent warps with lane refill: lanes whose
 // Levenberg-Marquardt solve has returned finish their pair and take the next one from a
-// global queue.  order (optional): the first pass takes the pairs in that order (the queue
-// order above); hist (optional): each pair's outcome is recorded there for the next
+// global queue.  order (optional): the first pass takes the *npairs pairs of that order (the
+// queue order above, tested for separation); hist (optional): each pair's outcome is recorded there for the next
 // collision phase's order.
 //
 // Finishing and taking a pair cost about as much as a step, with only the lanes that do
@@ -174,6 +183,11 @@ void launch_queue_order(const InstDev *insts, const PoolView *pv, const PairRec 
 // kernel (`in` set) resumes those solves under a larger budget or none.  The iterates are
 // the same operations in the same order.
 constexpr int kContactService = 8;
+// With the pairs in order, up to kSoloUpTo of them a warp, the first warp of every block
+// takes a single one, among them the longest, and the other three share the rest: the phase
+// then ends with lone solves (1 M spheroids 0.222 -> 0.209 ms, 1.5 M 0.271 -> 0.226; with
+// full warps the lost lanes cost more than the lone solves gain: 200,000 packed and more).
+constexpr int kSoloUpTo = 16;
 
 __global__ void __launch_bounds__(128, 2) k_contact(const InstDev *__restrict__ insts,
                                                     const PoolView *__restrict__ pv,
@@ -195,8 +209,12 @@ __global__ void __launch_bounds__(128, 2) k_contact(const InstDev *__restrict__ 
   constexpr unsigned kFull = 0xffffffffu;
   // lanes of a warp that take pairs: as few as cover the pairs with every warp in use
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  const unsigned per = (unsigned)min((int64_t)32, max((int64_t)1, (np + warps - 1) / warps));
-  const bool takes = lane < per;
+  const int64_t blocks = gridDim.x, rank = threadIdx.x >> 5;
+  int64_t solo = blocks;                       // pairs that have a warp to themselves
+  int64_t per = np <= warps ? 1 : (np - solo + (warps - blocks) - 1) / (warps - blocks);
+  if (per > kSoloUpTo) { solo = 0; per = min((int64_t)32, (np + warps - 1) / warps); }
+  const unsigned mine = solo && rank == 0 ? 1u : (unsigned)per;
+  const bool takes = lane < mine;
   bool active = false, done = false, exhausted = false;
   // Each warp's first batch is fixed: warp w of block b takes batch w * gridDim.x + b of
   // the ordered pairs, so that every block holds one warp of the longest solves, one of
@@ -220,12 +238,16 @@ __global__ void __launch_bounds__(128, 2) k_contact(const InstDev *__restrict__ 
         const unsigned want = __ballot_sync(kFull, takes && !active);
         unsigned long long base = 0;
         if (fixed) {
-          base = ((unsigned long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * per;
+          // batch `rank` of the block: the solo pairs first, then `per` pairs a warp
+          base = solo ? (rank == 0 ? (unsigned long long)blockIdx.x
+                                   : (unsigned long long)(blocks + ((rank - 1) * blocks + blockIdx.x) * per))
+                      : (unsigned long long)((rank * blocks + blockIdx.x) * per);
           fixed = false;
         } else {
           const int leader = __ffs(want) - 1;
           if ((int)lane == leader) base = atomicAdd(queue, (unsigned long long)__popc(want));
-          base = __shfl_sync(kFull, base, leader) + (unsigned long long)warps * per;
+          base = __shfl_sync(kFull, base, leader) +
+                 (unsigned long long)(solo ? blocks + (warps - blocks) * per : warps * per);
         }
         if ((int64_t)base >= np) {
           exhausted = true;
@@ -239,13 +261,11 @@ __global__ void __launch_bounds__(128, 2) k_contact(const InstDev *__restrict__ 
               active = true;
             } else {
               e = order ? (int64_t)order[q] : q;
-              active = take_pair(insts, pv, pairs, e, cp, s);
+              active = take_pair(insts, pv, pairs, e, order != nullptr, cp, s);
             }
             if (active) {
               CP = cp;
               S = s;
-            } else if (hist) {
-              record_apart(insts, pv, pairs, e, hist, nhist);
             }
           }
         }

@@ -261,7 +261,6 @@ int make_field_map(const void* field, int nx, int ny, int nz, CUtensorMap* out) 
 void launch_gather_tma(const CUtensorMap& map, const InstDev* insts, const PoolView* pv, const int32_t* perm,
                        int64_t n, double* const* fluid, unsigned long long* ticket, Status* st, int grid,
                        cudaStream_t s) {
-  cudaMemsetAsync(ticket, 0, sizeof(unsigned long long), s);
   k_gather_tma<<<grid, kTmaThreads, kTmaSmemBytes, s>>>(map, insts, pv, perm, n, fluid, ticket, st);
 }
 

@@ -11,30 +11,32 @@
 namespace gp {
 
 template __global__ void k_integrate<false>(const InstDev *, const PoolView *, const PoolView *, const int32_t *,
-                                            int64_t, const double *const *, uint32_t *, Status *);
+                                            int64_t, const double *const *, uint32_t *, PoolView *, PoolView *,
+                                            unsigned long long *, unsigned long long *, Status *);
 template __global__ void k_integrate_fix<false>(const InstDev *, const PoolView *, const PoolView *, const PairRec *,
                                                 const unsigned long long *, int64_t, const double *const *,
-                                                uint32_t *, Status *);
+                                                uint32_t *, PoolView *, PoolView *, unsigned long long *,
+                                                unsigned long long *, Status *);
 template __global__ void k_gather<false>(const InstDev *, const PoolView *, const int32_t *, int64_t, int,
                                          double *const *, unsigned long long *, Status *);
 
 void launch_gather_fp64(const InstDev *insts, const PoolView *pv, const int32_t *perm, int64_t n,
                       double *const *fluid, unsigned long long *ticket, Status *st, int grid, cudaStream_t s) {
-  cudaMemsetAsync(ticket, 0, sizeof(unsigned long long), s);
   k_gather<false><<<grid, 256, 0, s>>>(insts, pv, perm, n, gather_run(n), fluid, ticket, st);
 }
 
 void launch_integrate_fp64(const InstDev *insts, PoolView *pv, PoolView *pv_alt, const int32_t *perm, int64_t n,
-                         double *const *fluid, Status *st, int grid, cudaStream_t s, uint32_t *mark) {
-  k_integrate<false><<<grid, 128, 0, s>>>(insts, pv, pv_alt, perm, n, fluid, mark, st);
-  if (mark == nullptr) k_swap_pool<<<1, 1, 0, s>>>(pv, pv_alt, st);
+                         double *const *fluid, Status *st, int grid, unsigned long long *done,
+                         unsigned long long *ticket, cudaStream_t s, uint32_t *mark) {
+  k_integrate<false><<<grid, 128, 0, s>>>(insts, pv, pv_alt, perm, n, fluid, mark, pv, pv_alt, done, ticket, st);
 }
 
 void launch_integrate_fix_fp64(const InstDev *insts, PoolView *pv, PoolView *pv_alt, const PairRec *pairs,
                              const unsigned long long *npairs, int64_t cap_pairs, double *const *fluid,
-                             uint32_t *mark, Status *st, int grid, cudaStream_t s) {
-  k_integrate_fix<false><<<grid, 128, 0, s>>>(insts, pv, pv_alt, pairs, npairs, cap_pairs, fluid, mark, st);
-  k_swap_pool<<<1, 1, 0, s>>>(pv, pv_alt, st);
+                             uint32_t *mark, Status *st, int grid, unsigned long long *done,
+                             unsigned long long *ticket, cudaStream_t s) {
+  k_integrate_fix<false><<<grid, 128, 0, s>>>(insts, pv, pv_alt, pairs, npairs, cap_pairs, fluid, mark, pv, pv_alt,
+                                              done, ticket, st);
 }
 
 // INTERP_LAG3 (interp_lag3.f90:11-298) for one component at arbitrary points.
@@ -199,10 +201,10 @@ __global__ void k_point_order(int64_t n, const uint32_t *__restrict__ key, const
 static int point_grid(int64_t n) { return (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16); }
 
 void launch_point_order(const InstDev *inst, int64_t n, int shift, int64_t bins, const double *x, const double *y,
-                        const double *z, uint32_t *key, int32_t *count, int32_t *start, int32_t *scan_tmp,
-                        int32_t *order, cudaStream_t s) {
+                        const double *z, uint32_t *key, int32_t *count, int32_t *start,
+                        unsigned long long *state, int32_t *order, Status *st, cudaStream_t s) {
   k_point_bins<<<point_grid(n), 256, 0, s>>>(inst, n, shift, x, y, z, key, count);
-  launch_scan(count, start, bins, scan_tmp, nullptr, s);
+  launch_scan(count, start, bins, state, nullptr, st, s);
   k_point_order<<<point_grid(n), 256, 0, s>>>(n, key, start, count, order);
 }
 

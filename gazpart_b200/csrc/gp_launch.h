@@ -12,24 +12,27 @@ struct TailRec;   // gp_contact.cuh
 
 // --- gp_kernels_fp64.cu (FP64 path, -fmad=false) ---
 // ADV_PARTICLE_ELLP: advances particle perm[j] of *pv into slot j of *pv_alt, then swaps
-// the two views (so *pv is current afterwards).  With mark non-null, the speculative
-// pass: marked particles are left to launch_integrate_fix_*, which also swaps.
+// the two views (so *pv is current afterwards) and takes the gather's ticket back to zero.
+// With mark non-null, the speculative pass: marked particles are left to
+// launch_integrate_fix_*, which does both.  done: a counter, zero between launches.
 void launch_gather_fp64(const InstDev *insts, const PoolView *pv, const int32_t *perm, int64_t n,
                       double *const *fluid, unsigned long long *ticket, Status *st, int grid, cudaStream_t s);
 void launch_integrate_fp64(const InstDev *insts, PoolView *pv, PoolView *pv_alt, const int32_t *perm, int64_t n,
-                         double *const *fluid, Status *st, int grid, cudaStream_t s, uint32_t *mark = nullptr);
+                         double *const *fluid, Status *st, int grid, unsigned long long *done,
+                         unsigned long long *ticket, cudaStream_t s, uint32_t *mark = nullptr);
 void launch_integrate_fix_fp64(const InstDev *insts, PoolView *pv, PoolView *pv_alt, const PairRec *pairs,
                              const unsigned long long *npairs, int64_t cap_pairs, double *const *fluid,
-                             uint32_t *mark, Status *st, int grid, cudaStream_t s);
+                             uint32_t *mark, Status *st, int grid, unsigned long long *done,
+                             unsigned long long *ticket, cudaStream_t s);
 // order (or null): the indices of the points in the order to take them, as
 // launch_point_order leaves them (bins: rows of mesh cells cut into runs of 2^shift cells,
-// ny * nz * ((nx >> shift) + 1) of them; count: bins + 1 zeros;
-// start: bins + 1; scan_tmp: scan_block_sums_size(bins); key, order: n).
+// ny * nz * ((nx >> shift) + 1) of them; count: bins + 1 zeros; start: bins + 1; state:
+// scan_tiles(bins) zeros; key, order: n).
 void launch_interp(const InstDev *inst, bool mixed, int comp, int64_t n, const int32_t *order, const double *x,
                    const double *y, const double *z, double *out, Status *st, cudaStream_t s);
 void launch_point_order(const InstDev *inst, int64_t n, int shift, int64_t bins, const double *x, const double *y,
-                        const double *z, uint32_t *key, int32_t *count, int32_t *start, int32_t *scan_tmp,
-                        int32_t *order, cudaStream_t s);
+                        const double *z, uint32_t *key, int32_t *count, int32_t *start,
+                        unsigned long long *state, int32_t *order, Status *st, cudaStream_t s);
 void launch_frozen_interp(const double *xain, const double *yain, const double *zain, int nx, int ny, int nz,
                           const double *uain, int64_t n, const double *x, const double *y, const double *z,
                           double *out, Status *st, cudaStream_t s);
@@ -41,12 +44,15 @@ void launch_contact(const InstDev *insts, const PoolView *pv, const PairRec *pai
                     unsigned long long *nout, int64_t cap_out, int budget, const uint32_t *order,
                     uint32_t *hist, int64_t nhist, Status *st, int grid, cudaStream_t s);
 size_t tail_record_bytes();
-// The contact queue's order for the candidate pairs (gp_contact.cu): bins holds
-// 2 * kQueueBins counters, zero at the launch; key one byte per pair slot.
+// The contact queue's order (gp_contact.cu): order[0, *nsolve) are the candidate pairs that
+// are not proven apart, longest predicted solve first; the record hist[0, nhist) is cleared
+// for this phase's solves.  bins holds 2 * kQueueBins counters, zero at the launch; key one
+// byte per pair slot.
 constexpr int kQueueBins = 256;
 void launch_queue_order(const InstDev *insts, const PoolView *pv, const PairRec *pairs,
-                        const unsigned long long *npairs, int64_t cap_pairs, const uint32_t *hist, int64_t nhist,
-                        uint8_t *key, uint32_t *bins, uint32_t *order, const Status *st, int grid, cudaStream_t s);
+                        const unsigned long long *npairs, int64_t cap_pairs, uint32_t *hist, int64_t nhist,
+                        uint8_t *key, uint32_t *bins, uint32_t *order, unsigned long long *nsolve, const Status *st,
+                        int grid, cudaStream_t s);
 void launch_response(const InstDev *insts, const PoolView *pv, const CollRec *coll, const unsigned long long *ncoll,
                      int64_t cap_coll, const int8_t *state, int32_t *acc_list, unsigned long long *nacc, Status *st,
                      int grid, cudaStream_t s);
@@ -91,18 +97,32 @@ void launch_collision_stats(const CollRec *coll, const unsigned long long *ncoll
 void launch_gather_mixed(const InstDev *insts, const PoolView *pv, const int32_t *perm, int64_t n,
                       double *const *fluid, unsigned long long *ticket, Status *st, int grid, cudaStream_t s);
 void launch_integrate_mixed(const InstDev *insts, PoolView *pv, PoolView *pv_alt, const int32_t *perm, int64_t n,
-                         double *const *fluid, Status *st, int grid, cudaStream_t s, uint32_t *mark = nullptr);
+                         double *const *fluid, Status *st, int grid, unsigned long long *done,
+                         unsigned long long *ticket, cudaStream_t s, uint32_t *mark = nullptr);
 void launch_integrate_fix_mixed(const InstDev *insts, PoolView *pv, PoolView *pv_alt, const PairRec *pairs,
                              const unsigned long long *npairs, int64_t cap_pairs, double *const *fluid,
-                             uint32_t *mark, Status *st, int grid, cudaStream_t s);
+                             uint32_t *mark, Status *st, int grid, unsigned long long *done,
+                             unsigned long long *ticket, cudaStream_t s);
 void launch_iota(int32_t *a, int64_t n, cudaStream_t s);
 
 // --- gp_search.cu ---
+// What k_bin_count clears for the phases after it.
+struct PhaseClear {
+  unsigned long long *counters;     // those of the first ncounters (at most 32) in counter_mask
+  unsigned counter_mask;
+  int ncounters;
+  uint32_t *bins;                   // or null
+  int nbins;
+  unsigned long long *tile_state;   // the scan's
+  int64_t tiles;
+};
 void launch_bin_count(const InstDev *insts, const PoolView *pv, int64_t n, SearchArrays sa, Status *st, int grid,
-                      cudaStream_t s);
-// (clears clear[0..n) on the way)
-void launch_scan(const int32_t *in, int32_t *out, int64_t n, int32_t *block_sums, float *clear, cudaStream_t s);
-int64_t scan_block_sums_size(int64_t n);
+                      const PhaseClear &clear, cudaStream_t s);
+// Exclusive scan of n counts; state: scan_tiles(n) words, zero at the launch; clears
+// clear[0..n] on the way where it is not null.
+int64_t scan_tiles(int64_t n);
+void launch_scan(const int32_t *in, int32_t *out, int64_t n, unsigned long long *state, float *clear, Status *st,
+                 cudaStream_t s);
 void launch_bin_scatter(const InstDev *insts, const PoolView *pv, int64_t n, SearchArrays sa, Status *st, int grid,
                         cudaStream_t s);
 void launch_search(const InstDev *insts, const PoolView *pv, int64_t n, SearchArrays sa, PairRec *pairs, unsigned long long *npairs,

@@ -73,11 +73,19 @@ __device__ __forceinline__ void cell_coords(const InstDev &I, int32_t cell, int 
   cy = t - cz * I.nfy;
 }
 
+// Also clears what the rest of the collision phase counts in (also in a step after a halted
+// one, whose scan and search still run): a clearing pass of its own costs a launch each.
 __global__ void k_bin_count(const InstDev *__restrict__ insts, const PoolView *__restrict__ pv, int64_t n,
-                            SearchArrays sa, const Status *st) {
+                            SearchArrays sa, PhaseClear clear, const Status *st) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, gid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  for (int64_t k = gid; k < clear.tiles; k += stride) clear.tile_state[k] = 0ull;
+  if (blockIdx.x == 0) {
+    if (threadIdx.x < clear.ncounters && (clear.counter_mask >> threadIdx.x) & 1u) clear.counters[threadIdx.x] = 0ull;
+    if (clear.bins != nullptr)
+      for (int k = threadIdx.x; k < clear.nbins; k += blockDim.x) clear.bins[k] = 0u;
+  }
   if (step_halted(st)) return;
   const PoolView P = *pv;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t nround = (n + stride - 1) / stride * stride;   // whole warps stay in the loop
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nround; i += stride) {
     int32_t c = -1;
@@ -100,20 +108,32 @@ __global__ void k_bin_count(const InstDev *__restrict__ insts, const PoolView *_
   }
 }
 
-void launch_bin_count(const InstDev *insts, const PoolView *pv, int64_t n, SearchArrays sa, Status *st,
-                      int grid, cudaStream_t s) {
-  k_bin_count<<<grid, 256, 0, s>>>(insts, pv, n, sa, st);
+void launch_bin_count(const InstDev *insts, const PoolView *pv, int64_t n, SearchArrays sa, Status *st, int grid,
+                      const PhaseClear &clear, cudaStream_t s) {
+  k_bin_count<<<grid, 256, 0, s>>>(insts, pv, n, sa, clear, st);
 }
 
 // ---------------------------------------------------------------------------
-// 2. exclusive scan (three-level, 2048 elements per block)
+// 2. exclusive scan, one pass
 // ---------------------------------------------------------------------------
+// Blocks take tiles of 2048 counts in order from a counter. A tile publishes its sum at once
+// and its inclusive prefix as soon as it has it; a block adds up the sums before its tile
+// back to the nearest prefix (the decoupled look-back of D. Merrill and M. Garland, NVIDIA
+// NVR-2016-002).  The tiles before a block's were taken by blocks that are running, so the
+// wait ends; it is bounded all the same.  One launch instead of three to five.
+// state[0] is the counter, state[1 + t] tile t: status (1 sum, 2 prefix) << 32 | value; all
+// zero at the launch.
 constexpr int kScanThreads = 512, kScanPer = 4, kScanBlock = kScanThreads * kScanPer;
 
-__global__ void k_scan_block(const int32_t *__restrict__ in, int32_t *__restrict__ out, int64_t n,
-                             int32_t *__restrict__ sums, float *__restrict__ clear) {
+__global__ void __launch_bounds__(kScanThreads) k_scan(const int32_t *__restrict__ in, int32_t *__restrict__ out,
+                                                       int64_t n, unsigned long long *state,
+                                                       float *__restrict__ clear, Status *st) {
   __shared__ int32_t warp_tot[kScanThreads / 32];
-  const int64_t base = (int64_t)blockIdx.x * kScanBlock + (int64_t)threadIdx.x * kScanPer;
+  __shared__ int64_t tile_s;
+  __shared__ int32_t before_s;
+  if (threadIdx.x == 0) tile_s = (int64_t)atomicAdd(&state[0], 1ull);
+  __syncthreads();
+  const int64_t tile = tile_s, base = tile * kScanBlock + (int64_t)threadIdx.x * kScanPer;
   int32_t v[kScanPer];
   int32_t run = 0;
 #pragma unroll
@@ -142,9 +162,36 @@ __global__ void k_scan_block(const int32_t *__restrict__ in, int32_t *__restrict
       if (lane >= o) w += y;
     }
     if (lane < kScanThreads / 32) warp_tot[lane] = w;
+    const int32_t total = __shfl_sync(0xffffffffu, w, kScanThreads / 32 - 1);
+    volatile unsigned long long *tiles = state + 1;
+    if (lane == 0) tiles[tile] = ((tile == 0 ? 2ull : 1ull) << 32) | (unsigned)total;
+    int32_t before = 0;
+    if (tile > 0) {
+      // look back 32 tiles at a time, lane 0 at the nearest
+      int64_t at = tile - 1;
+      for (int spin = 0;;) {
+        const int64_t k = at - lane;
+        const unsigned long long e = k >= 0 ? tiles[k] : (2ull << 32);
+        const int status = (int)(e >> 32);
+        if (__any_sync(0xffffffffu, status == 0)) {
+          if (++spin > (1 << 24)) {   // cannot happen
+            if (lane == 0) set_error(st, GP_ETIMEOUT, tile);
+            break;
+          }
+          continue;
+        }
+        const unsigned whole = __ballot_sync(0xffffffffu, status == 2);
+        const int last = whole ? __ffs(whole) - 1 : 31;   // the nearest prefix ends the sum
+        before += __reduce_add_sync(0xffffffffu, lane <= last ? (int32_t)(unsigned)e : 0);
+        if (whole) break;
+        at -= 32;
+      }
+      if (lane == 0) tiles[tile] = (2ull << 32) | (unsigned)(before + total);
+    }
+    if (lane == 0) before_s = before;
   }
   __syncthreads();
-  const int32_t excl = x - run + (wid > 0 ? warp_tot[wid - 1] : 0);
+  const int32_t excl = before_s + x - run + (wid > 0 ? warp_tot[wid - 1] : 0);
 #pragma unroll
   for (int k = 0; k < kScanPer; ++k) {
     const int64_t idx = base + k;
@@ -153,41 +200,15 @@ __global__ void k_scan_block(const int32_t *__restrict__ in, int32_t *__restrict
       if (clear != nullptr) clear[idx] = 0.f;
     }
   }
-  if (threadIdx.x == kScanThreads - 1 && sums != nullptr) sums[blockIdx.x] = excl + run;
 }
 
-__global__ void k_scan_add(int32_t *__restrict__ out, int64_t n, const int32_t *__restrict__ offs) {
-  const int64_t base = (int64_t)blockIdx.x * kScanBlock;
-  const int32_t o = offs[blockIdx.x];
-  for (int k = threadIdx.x; k < kScanBlock; k += blockDim.x) {
-    const int64_t idx = base + k;
-    if (idx < n) out[idx] += o;
-  }
-}
-
-static int64_t nblocks(int64_t n) { return (n + kScanBlock - 1) / kScanBlock; }
-
-int64_t scan_block_sums_size(int64_t n) {
-  // level-1 sums, level-2 sums (and their scans)
-  const int64_t b1 = nblocks(n + 1), b2 = nblocks(b1), b3 = nblocks(b2);
-  return 2 * (b1 + b2 + b3) + 16;
-}
+int64_t scan_tiles(int64_t n) { return (n + 1 + kScanBlock - 1) / kScanBlock + 1; }
 
 // out[0..n] = exclusive scan of in[0..n-1], out[n] = total.  in[n] must be readable
 // as zero (the caller allocates n+1 counters, and n+1 values of clear).
-void launch_scan(const int32_t *in, int32_t *out, int64_t n, int32_t *tmp, float *clear, cudaStream_t s) {
-  const int64_t m = n + 1;
-  const int64_t b1 = nblocks(m), b2 = nblocks(b1), b3 = nblocks(b2);
-  int32_t *s1 = tmp, *s1x = s1 + b1, *s2 = s1x + b1, *s2x = s2 + b2, *s3 = s2x + b2;
-  k_scan_block<<<(unsigned)b1, kScanThreads, 0, s>>>(in, out, m, s1, clear);
-  if (b1 > 1) {
-    k_scan_block<<<(unsigned)b2, kScanThreads, 0, s>>>(s1, s1x, b1, s2, nullptr);
-    if (b2 > 1) {
-      k_scan_block<<<(unsigned)b3, kScanThreads, 0, s>>>(s2, s2x, b2, s3, nullptr);   // b3 == 1 for n < 8.6e9
-      k_scan_add<<<(unsigned)b2, kScanThreads, 0, s>>>(s1x, b1, s2x);
-    }
-    k_scan_add<<<(unsigned)b1, kScanThreads, 0, s>>>(out, m, s1x);
-  }
+void launch_scan(const int32_t *in, int32_t *out, int64_t n, unsigned long long *state, float *clear, Status *st,
+                 cudaStream_t s) {
+  k_scan<<<(unsigned)(scan_tiles(n) - 1), kScanThreads, 0, s>>>(in, out, n + 1, state, clear, st);
 }
 
 // ---------------------------------------------------------------------------
