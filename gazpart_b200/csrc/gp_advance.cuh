@@ -407,11 +407,26 @@ __device__ __forceinline__ void k_omega(const double t[3], double ox, double oy,
   }
 }
 
+// mult_quat with the multiply-adds named, so that the compiler fuses none of its own choice;
+// kPredictor: the rounding of the first two products of b and d in the predictor's step is
+// the other way round than in the corrector's (either is as good; both are kept so
+// that the results stay the same bits).
+template <bool kPredictor>
+__device__ __forceinline__ Quat mult_quat_fused(const Quat& x, const Quat& y) {
+  const double b = kPredictor ? __fma_rn(x.b, y.a, __dmul_rn(x.a, y.b)) : __fma_rn(x.a, y.b, __dmul_rn(x.b, y.a));
+  const double d = kPredictor ? __fma_rn(x.b, y.c, __dmul_rn(x.a, y.d)) : __fma_rn(x.a, y.d, __dmul_rn(x.b, y.c));
+  return {__fma_rn(-x.d, y.d, __fma_rn(-x.c, y.c, __fma_rn(x.a, y.a, __dmul_rn(-x.b, y.b)))),
+          __fma_rn(-x.d, y.c, __fma_rn(x.c, y.d, b)),
+          __fma_rn(x.d, y.b, __fma_rn(x.c, y.a, __fma_rn(x.a, y.c, __dmul_rn(-x.b, y.d)))),
+          __fma_rn(x.d, y.a, __fma_rn(-x.c, y.b, d))};
+}
+
 // Quaternion step of adv_quaternion.f90:39-84 followed by renormalisation (mixed form).
 // r = R(q) in FP32: the body-to-lab rotation that the stage's force evaluation already
 // built.  The increment (the spin in the lab frame, the half angle's sine and cosine) is
 // FP32: a relative error of a few 1e-8 of one step's rotation; the product with q and
 // the renormalisation are FP64.
+template <bool kPredictor>
 __device__ __forceinline__ void quaternion_step_mixed(Quat& q, const float r[9], double ox, double oy, double oz,
                                                       double dt) {
   const float w0 = (float)ox, w1 = (float)oy, w2 = (float)oz;
@@ -446,15 +461,16 @@ __device__ __forceinline__ void quaternion_step_mixed(Quat& q, const float r[9],
     const float si = __fmul_rn(s, inv);
     map = {(double)c, (double)__fmul_rn(si, g0), (double)__fmul_rn(si, g1), (double)__fmul_rn(si, g2)};
   }
-  q = mult_quat(map, q);
-  const double inv = rsqrt(q.a * q.a + q.b * q.b + q.c * q.c + q.d * q.d);
-  q.a *= inv; q.b *= inv; q.c *= inv; q.d *= inv;
+  q = mult_quat_fused<kPredictor>(map, q);
+  const double inv =
+      rsqrt(__fma_rn(q.d, q.d, __fma_rn(q.c, q.c, __fma_rn(q.a, q.a, __dmul_rn(q.b, q.b)))));
+  q.a = __dmul_rn(q.a, inv); q.b = __dmul_rn(q.b, inv); q.c = __dmul_rn(q.c, inv); q.d = __dmul_rn(q.d, inv);
 }
 
 // One quaternion update; r = R(q) is used by the mixed form only.
-template <bool kMixed>
+template <bool kMixed, bool kPredictor = false>
 __device__ __forceinline__ void quat_advance(Quat& q, const float r[9], double ox, double oy, double oz, double dt) {
-  if (kMixed) quaternion_step_mixed(q, r, ox, oy, oz, dt);
+  if (kMixed) quaternion_step_mixed<kPredictor>(q, r, ox, oy, oz, dt);
   else quaternion_integration(q, ox, oy, oz, dt);
 }
 
@@ -515,7 +531,7 @@ __device__ __forceinline__ int advance_particle(const InstDev& I, const PartCons
   double u1[3] = {U[0] + dt * k1u[0], U[1] + dt * k1u[1], U[2] + dt * k1u[2]};
   double o1[3] = {O[0] + dt * k1o[0], O[1] + dt * k1o[1], O[2] + dt * k1o[2]};
   Quat q1 = Q;
-  quat_advance<kMixed>(q1, r0, o1[0], o1[1], o1[2], dt);
+  quat_advance<kMixed, true>(q1, r0, o1[0], o1[1], o1[2], dt);
   double wn[3], arm[3], delta_x = 0.0;
   bool isect;
   int rc = wall_test_adv<kMixed>(I.lx, pc, S, si, rmax, xp1, yp1, zp1, q1, wn, arm, delta_x, isect);
@@ -854,18 +870,116 @@ __global__ void __launch_bounds__(256, GP_GATHER_MIN_BLOCKS) k_gather(const Inst
   }
 }
 
-// advance_particle where the straight-line step gave up (FP64 form).  Out of line, on
-// copies, so that the state of the common path stays in registers.
+// advance_particle for the particles that the slot steps leave to it (an intersected wall,
+// an error, FP64 operands out of the straight line's range): from the pool, out of line.
 struct StepState {
   double X[3], U[3], O[3];
   Quat Q;
 };
-static __device__ __noinline__ int advance_particle_general(const InstDev* I, const PoolView* S, int64_t si,
+template <bool kMixed>
+static __device__ __noinline__ int advance_particle_general(const InstDev* I, const PoolView* S, int64_t i,
                                                             const double* fluid, StepState* s) {
+  const PoolView& P = *S;
   PartConst pc;
-  load_pc(*S, si, pc);
+  load_pc(P, i, pc);
   MixedConst mc;
-  return advance_particle<false>(*I, pc, mc, *S, si, fluid, fluid + 3, s->X, s->U, s->O, s->Q);
+  if (kMixed) mixed_const(pc, I->visc, mc);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) { s->X[k] = P.st[k][i]; s->U[k] = P.st[3 + k][i]; s->O[k] = P.st[10 + k][i]; }
+  s->Q = {P.st[6][i], P.st[7][i], P.st[8][i], P.st[9][i]};
+  return advance_particle<kMixed>(*I, pc, mc, P, i, fluid, fluid + 3, s->X, s->U, s->O, s->Q);
+}
+
+// advance_particle<true> where no wall is intersected and no error met; false: not done.
+// The slot's quaternion and constant columns are overwritten (k1u, k1o and the four
+// constants that stay FP64).  The FP64 operations name their roundings, so that the compiler
+// fuses none of its own choice.
+GP_LF bool advance_mixed_slot(const InstDev& I, const Slot& a, const PoolView& S, int64_t si, double xn[3],
+                              double un[3], double on[3], Quat& qn) {
+  const double dt = I.dtime;
+  MixedConst mc;
+  {
+    PartConst pc;
+    a.get_const(pc);
+    mixed_const(pc, I.visc, mc);
+  }
+  constexpr int kDiff = kSlotConst + 6;   // dyz, dzx, dxy, rmax
+  a.put(kDiff, mc.dyz); a.put(kDiff + 1, mc.dzx); a.put(kDiff + 2, mc.dxy); a.put(kDiff + 3, mc.rmax);
+  auto spin_rate = [&](const double t[3], const double o[3], double k[3]) {
+    k[0] = __dmul_rn(__fma_rn(__dmul_rn(o[1], o[2]), a.get(kDiff), t[0]), (double)mc.rix);
+    k[1] = __dmul_rn(__fma_rn(__dmul_rn(o[2], o[0]), a.get(kDiff + 1), t[1]), (double)mc.riy);
+    k[2] = __dmul_rn(__fma_rn(__dmul_rn(o[0], o[1]), a.get(kDiff + 2), t[2]), (double)mc.riz);
+  };
+  auto at_wall = [&](double x, double y, double z, const Quat& q) {
+    if (off_wall(I.lx, a.get(kDiff + 3), x)) return false;
+    PartConst c;
+    load_pc(S, si, c);
+    const Quat qq = q;
+    return wall_hit(I.lx, &c, x, y, z, &qq);
+  };
+  double f[3], t[3], o[3], k1[3];
+  float r[9];
+  Quat q1 = a.quat();
+  rotmat_f(q1, r);
+  {
+    RelFlow q;
+    double u[3], uf[3], wv[3];
+    a.get3(kSlotU, u);
+    a.get3(kSlotFluid, uf);
+    rel_flow(mc, u, uf, r, q);
+    if (!fluid_force_mixed(mc, q, r, f)) return false;
+    f[2] = f[2] + I.gravity;
+    a.put3(kSlotConst, f);
+    a.get3(kSlotFluid + 3, wv);
+    a.get3(kSlotO, o);
+    if (o[0] != o[0]) return false;
+    fluid_torque_mixed(mc, q, wv, o[0], o[1], o[2], r, t);
+    spin_rate(t, o, k1);
+    a.put3(kSlotConst + 3, k1);
+  }
+  auto predicted = [&](int col, int rate, double v[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) v[i] = __dadd_rn(a.get(col + i), __dmul_rn(dt, a.get(rate + i)));
+  };
+  predicted(kSlotO, kSlotConst + 3, o);
+  quaternion_step_mixed<true>(q1, r, o[0], o[1], o[2], dt);
+  if (at_wall(a.get(0) + dt * a.get(3), a.get(1) + dt * a.get(4), a.get(2) + dt * a.get(5), q1)) return false;
+  a.put_quat(q1);
+  rotmat_f(q1, r);
+  {
+    RelFlow q;
+    double u[3], uf[3], wv[3];
+    predicted(kSlotU, kSlotConst, u);
+    a.get3(kSlotFluid, uf);
+    rel_flow(mc, u, uf, r, q);
+    if (!fluid_force_mixed(mc, q, r, f)) return false;
+    a.get3(kSlotU, u);
+    a.get3(kSlotFluid, uf);
+    rel_flow(mc, u, uf, r, q);
+    a.get3(kSlotFluid + 3, wv);
+    predicted(kSlotO, kSlotConst + 3, o);
+    if (o[0] != o[0]) return false;
+    fluid_torque_mixed(mc, q, wv, o[0], o[1], o[2], r, t);
+  }
+  double k2o[3];
+  spin_rate(t, o, k2o);
+  const double h = __dmul_rn(0.5, dt), k2u[3] = {f[0], f[1], f[2] + I.gravity};
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const double u = a.get(kSlotU + i), k1u = a.get(kSlotConst + i), u1 = __dadd_rn(u, __dmul_rn(dt, k1u));
+    xn[i] = __dadd_rn(a.get(i), __dmul_rn(h, __dadd_rn(u, u1)));
+    un[i] = __dadd_rn(u, __dmul_rn(h, __dadd_rn(k1u, k2u[i])));
+    on[i] = __dadd_rn(a.get(kSlotO + i), __dmul_rn(h, __dadd_rn(a.get(kSlotConst + 3 + i), k2o[i])));
+  }
+  qn = a.quat();
+  if (at_wall(xn[0], xn[1], xn[2], qn)) return false;
+  quaternion_step_mixed<false>(qn, r, on[0], on[1], on[2], dt);
+  return true;
+}
+
+// A particle's columns on their way into its slot.
+__device__ __forceinline__ void copy_async8(unsigned to, const double* from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(from) : "memory");
 }
 
 // ADV_PARTICLE_ELLP, second half, for one particle: particle i of the source buffer is
@@ -875,39 +989,39 @@ static __device__ __noinline__ int advance_particle_general(const InstDev* I, co
 // BOUNDARY_PARTICLE's periodic wrap (boundary_particle.f90:50-59).  A particle whose
 // stencil left the field (NaN fluid values, reported by the gather) is copied unchanged.
 template <bool kMixed>
-__device__ __forceinline__ void integrate_slot(const InstDev* __restrict__ insts, const PoolView* __restrict__ S,
-                                               const PoolView* __restrict__ D, int64_t i, int64_t j,
-                                               const double* const* __restrict__ fluid, Status* st) {
-  const int inst = S->inst[i];
-  D->inst[j] = inst;
-  D->id[j] = S->id[i];
-  PartConst pc;
-  load_pc(*S, i, pc);
-#pragma unroll 1
-  for (int c = 0; c < kNConst; ++c) D->pc[c][j] = S->pc[c][i];
-  MixedConst mc;
-  double X[3] = {S->st[0][i], S->st[1][i], S->st[2][i]};
-  double U[3] = {S->st[3][i], S->st[4][i], S->st[5][i]};
-  Quat Q = {S->st[6][i], S->st[7][i], S->st[8][i], S->st[9][i]};
-  double O[3] = {S->st[10][i], S->st[11][i], S->st[12][i]};
-  const double uf[3] = {fluid[0][j], fluid[1][j], fluid[2][j]};
-  const double wv[3] = {fluid[3][j], fluid[4][j], fluid[5][j]};
+__device__ __forceinline__ void integrate_slot(const InstDev* __restrict__ insts, const PoolView& S, const PoolView& D,
+                                               int64_t i, int64_t j, const double* const* fluid, const Slot& a,
+                                               Status* st) {
+#pragma unroll
+  for (int k = 0; k < kNState; ++k) copy_async8(a.at + k * (kIntegrateThreads * 8), S.st[k] + i);
+#pragma unroll
+  for (int k = 0; k < kNConst; ++k) copy_async8(a.at + (kSlotConst + k) * (kIntegrateThreads * 8), S.pc[k] + i);
+#pragma unroll
+  for (int k = 0; k < kNFluid; ++k) copy_async8(a.at + (kSlotFluid + k) * (kIntegrateThreads * 8), fluid[k] + j);
+  const int inst = S.inst[i];
+  D.inst[j] = inst;
+  D.id[j] = S.id[i];
+  asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+  for (int k = 0; k < kNConst; ++k) D.pc[k][j] = a.get(kSlotConst + k);
+  double X[3], U[3], O[3];
+  Quat Q;
+  const double uf0 = a.get(kSlotFluid), wv0 = a.get(kSlotFluid + 3);
   // stencil out of range (reported by the gather): carried over unchanged
-  if (inst >= 0 && !(uf[0] != uf[0] && wv[0] != wv[0])) {
+  if (inst >= 0 && !(uf0 != uf0 && wv0 != wv0)) {
     const InstDev& I = insts[inst];
-    int err = 0;
-    if (kMixed) {
-      mixed_const(pc, I.visc, mc);
-      err = advance_particle<kMixed>(I, pc, mc, *S, i, uf, wv, X, U, O, Q);
-    } else if (!advance_particle_fast(I, pc, uf, wv, X, U, O, Q)) {
-      const double fl[6] = {uf[0], uf[1], uf[2], wv[0], wv[1], wv[2]};
-      StepState s = {{X[0], X[1], X[2]}, {U[0], U[1], U[2]}, {O[0], O[1], O[2]}, Q};
-      err = advance_particle_general(&I, S, i, fl, &s);
+    const bool done = kMixed ? advance_mixed_slot(I, a, S, i, X, U, O, Q) : advance_particle_fast(I, a, X, U, O, Q);
+    if (!done) {
+      double fl[6];
+      a.get3(kSlotFluid, fl);
+      a.get3(kSlotFluid + 3, fl + 3);
+      StepState s;
+      const int err = advance_particle_general<kMixed>(&I, &S, i, fl, &s);
+      if (err) set_error(st, err, (long long)S.id[i], inst);
 #pragma unroll
       for (int k = 0; k < 3; ++k) { X[k] = s.X[k]; U[k] = s.U[k]; O[k] = s.O[k]; }
       Q = s.Q;
     }
-    if (err) set_error(st, err, (long long)S->id[i], inst);
     // adv_particle_new.f90:685-686: the channel wraps y and z only
     // (boundary_particle_yz.f90:44-70), the others every direction when periodic
     if (I.frozen_flow == 3) {
@@ -923,11 +1037,34 @@ __device__ __forceinline__ void integrate_slot(const InstDev* __restrict__ insts
       if (X[2] > I.lz) X[2] = X[2] - I.lz;
       if (X[2] < 0.) X[2] = X[2] + I.lz;
     }
+  } else {
+    a.get3(kSlotX, X);
+    a.get3(kSlotU, U);
+    a.get3(kSlotO, O);
+    Q = a.quat();
   }
-  D->st[0][j] = X[0]; D->st[1][j] = X[1]; D->st[2][j] = X[2];
-  D->st[3][j] = U[0]; D->st[4][j] = U[1]; D->st[5][j] = U[2];
-  D->st[6][j] = Q.a; D->st[7][j] = Q.b; D->st[8][j] = Q.c; D->st[9][j] = Q.d;
-  D->st[10][j] = O[0]; D->st[11][j] = O[1]; D->st[12][j] = O[2];
+  D.st[0][j] = X[0]; D.st[1][j] = X[1]; D.st[2][j] = X[2];
+  D.st[3][j] = U[0]; D.st[4][j] = U[1]; D.st[5][j] = U[2];
+  D.st[6][j] = Q.a; D.st[7][j] = Q.b; D.st[8][j] = Q.c; D.st[9][j] = Q.d;
+  D.st[10][j] = O[0]; D.st[11][j] = O[1]; D.st[12][j] = O[2];
+}
+
+// The block's slots and the buffers' columns, in shared memory.
+template <bool kMixed>
+struct SlotBlock {
+  double v[kMixed ? kSlotIn : kSlotIn + 6][kIntegrateThreads];
+  PoolView from, to;
+  const double* fluid[kNFluid];
+};
+template <bool kMixed>
+__device__ __forceinline__ Slot open_slots(SlotBlock<kMixed>& b, const PoolView* src_pv, const PoolView* dst_pv,
+                                           const double* const* fluid) {
+  const int t = threadIdx.x;
+  if (t == 0) b.from = *src_pv;
+  if (t == 32) b.to = *dst_pv;
+  if (t >= 64 && t < 64 + kNFluid) b.fluid[t - 64] = fluid[t - 64];
+  __syncthreads();
+  return {(unsigned)__cvta_generic_to_shared(&b.v[0][t])};
 }
 
 // The end of an advance, by the last block to get here (the views are read by nobody any
@@ -953,23 +1090,33 @@ __device__ __forceinline__ void finish_advance(PoolView* a, PoolView* b, unsigne
 // alone: mark[i] receives j + 1 and k_integrate_fix advances it once the response is
 // done.  Unmarked particles are ones the response never touches, so both passes read
 // exactly the state a single pass after the response would read.
+//
+// What bounds it: 16 warps an SM, each in a chain of some 1,600 instructions; the step keeps
+// its state in shared memory (Slot) because the registers it spilled cost more than the
+// chain.  Measured (B200, one-step graphs): mixed 16.8 M particles 2.01 -> 1.59 ms (436
+// bytes a particle, 4.6 TB/s), 1 M 0.137 -> 0.117; FP64 1 M 0.298 -> 0.291.  Five and six
+// blocks per SM (96 and 80 registers): mixed 1.67 and 1.84, FP64 0.320 and 0.338.  Fetching a
+// particle's columns while the one before is advanced, with the state in registers, took
+// 2.11.
 #ifndef GP_INTEGRATE_MIN_BLOCKS
 #define GP_INTEGRATE_MIN_BLOCKS 4
 #endif
 template <bool kMixed>
-__global__ void __launch_bounds__(128, GP_INTEGRATE_MIN_BLOCKS)
+__global__ void __launch_bounds__(kIntegrateThreads, GP_INTEGRATE_MIN_BLOCKS)
     k_integrate(const InstDev* __restrict__ insts, const PoolView* __restrict__ src_pv,
                 const PoolView* __restrict__ dst_pv, const int32_t* __restrict__ perm, int64_t n,
                 const double* const* __restrict__ fluid, uint32_t* __restrict__ mark, PoolView* src, PoolView* dst,
                 unsigned long long* done, unsigned long long* ticket, Status* st) {
+  __shared__ SlotBlock<kMixed> b;
   if (step_halted(st)) return;
+  const Slot a = open_slots(b, src_pv, dst_pv, fluid);
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = perm[j];
     if (mark != nullptr && mark[i] != 0u) {
       mark[i] = (uint32_t)(j + 1);
       continue;
     }
-    integrate_slot<kMixed>(insts, src_pv, dst_pv, i, j, fluid, st);
+    integrate_slot<kMixed>(insts, b.from, b.to, i, j, b.fluid, a, st);
   }
   if (mark == nullptr) finish_advance(src, dst, done, ticket);
 }
@@ -979,19 +1126,21 @@ __global__ void __launch_bounds__(128, GP_INTEGRATE_MIN_BLOCKS)
 // first lane to clear its mark takes it), into the slot the speculative pass recorded.
 // The marks are all zero again afterwards.
 template <bool kMixed>
-__global__ void __launch_bounds__(128, GP_INTEGRATE_MIN_BLOCKS)
+__global__ void __launch_bounds__(kIntegrateThreads, GP_INTEGRATE_MIN_BLOCKS)
     k_integrate_fix(const InstDev* __restrict__ insts, const PoolView* __restrict__ src_pv,
                     const PoolView* __restrict__ dst_pv, const PairRec* __restrict__ pairs,
                     const unsigned long long* npairs, int64_t cap, const double* const* __restrict__ fluid,
                     uint32_t* __restrict__ mark, PoolView* src, PoolView* dst, unsigned long long* done,
                     unsigned long long* ticket, Status* st) {
+  __shared__ SlotBlock<kMixed> b;
   if (step_halted(st)) return;
+  const Slot a = open_slots(b, src_pv, dst_pv, fluid);
   const int64_t np = (int64_t)min(*npairs, (unsigned long long)cap);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 2 * np; e += (int64_t)gridDim.x * blockDim.x) {
     const PairRec& r = pairs[e >> 1];
     const int64_t i = (e & 1) ? r.near : r.home;
     const uint32_t v = atomicExch(&mark[i], 0u);
-    if (v != 0u) integrate_slot<kMixed>(insts, src_pv, dst_pv, i, (int64_t)v - 1, fluid, st);
+    if (v != 0u) integrate_slot<kMixed>(insts, b.from, b.to, i, (int64_t)v - 1, b.fluid, a, st);
   }
   finish_advance(src, dst, done, ticket);
 }

@@ -20,9 +20,7 @@
 // cosine 0.78 and 0.16 (CUDA's sincos 1.35 and 0.17); quotients and roots were equal to
 // CUDA's in every case.
 //
-// Measured (B200, integrate of one step): 1 M particles 0.58 -> 0.30 ms, 10,000 38 -> 21
-// us.  Four blocks of 128 per SM (128 registers, 480 B of spills) at 1 M: three take 0.42,
-// five 0.33.
+// Measured (B200, integrate of one step): 1 M particles 0.58 -> 0.30 ms, 10,000 38 -> 21 us.
 #pragma once
 #include "gp_lm_fast.cuh"
 
@@ -283,65 +281,133 @@ GP_LF void fw_quaternion(Quat& q, const double r[9], const double o[3], double d
   q = mult_quat(map, q);
 }
 
-// advance_particle<false> away from the walls.  False: not done (the state is unchanged).
-GP_LF bool advance_particle_fast(const InstDev& I, const PartConst& pc, const double uf[3], const double wv[3],
-                                 double X[3], double U[3], double O[3], Quat& Q) {
+// A particle on the way through the integrate: its columns in shared memory, one entry a
+// thread (nobody else's business, so no barriers), read again where they are needed instead
+// of kept in registers.  The step's own register file is too small for its state, and what
+// it spilled went through an L1 that the streamed columns kept flushing: 73 local loads a
+// particle, more than 100 cycles each.
+constexpr int kIntegrateThreads = 128;
+enum { kSlotX = 0, kSlotU = 3, kSlotQ = 6, kSlotO = 10, kSlotConst = 13, kSlotFluid = 23, kSlotWork = 29 };
+constexpr int kSlotIn = 29;      // columns read: 13 state, 10 constants, 6 fluid
+struct Slot {
+  unsigned at;                   // shared-memory address of column 0's entry
+  __device__ __forceinline__ double get(int k) const {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(at + k * (kIntegrateThreads * 8)));
+    return v;
+  }
+  __device__ __forceinline__ void put(int k, double v) const {
+    asm volatile("st.shared.f64 [%0], %1;" ::"r"(at + k * (kIntegrateThreads * 8)), "d"(v) : "memory");
+  }
+  __device__ __forceinline__ void get3(int k, double v[3]) const {
+    v[0] = get(k); v[1] = get(k + 1); v[2] = get(k + 2);
+  }
+  __device__ __forceinline__ void put3(int k, const double v[3]) const {
+    put(k, v[0]); put(k + 1, v[1]); put(k + 2, v[2]);
+  }
+  __device__ __forceinline__ Quat quat() const { return {get(kSlotQ), get(kSlotQ + 1), get(kSlotQ + 2), get(kSlotQ + 3)}; }
+  __device__ __forceinline__ void put_quat(const Quat& q) const {
+    put(kSlotQ, q.a); put(kSlotQ + 1, q.b); put(kSlotQ + 2, q.c); put(kSlotQ + 3, q.d);
+  }
+  __device__ __forceinline__ void get_const(PartConst& c) const {
+    c.a = get(13); c.b = get(14); c.deq = get(15); c.cdrag = get(16); c.cpitch = get(17);
+    c.crot = get(18); c.h5 = get(19); c.ipxx = get(20); c.ipyy = get(21); c.ipzz = get(22);
+  }
+};
+
+// Whether the body intersects its wall (or the test fails), for a centre within 1.5 radii
+// of it.  Out of line: few particles come here.
+static __device__ __noinline__ bool wall_hit(double lx, const PartConst* pc, double x, double y, double z,
+                                             const Quat* q) {
+  double wn[3], arm[3], dx;
+  bool isect;
+  return wall_test(lx, *pc, fmax(pc->a, pc->b), x, y, z, *q, wn, arm, dx, isect) != 0 || isect;
+}
+// wall_test's own early exit first.
+GP_LF bool off_wall(double lx, double rmax, double x) { return fabs(x - ((x < lx / 2.0) ? 0.0 : lx)) > 1.5 * rmax; }
+
+// advance_particle<false> away from the walls.  False: not done (the general step starts
+// from the pool again).  The slot's quaternion and work columns (six) are overwritten.
+GP_LF bool advance_particle_fast(const InstDev& I, const Slot& a, double xn[3], double un[3], double on[3], Quat& qn) {
   LfGuard g;
-  const double dt = I.dtime, rmax = fmax(pc.a, pc.b);
-  const LfRcp rv = lf_rcp(I.visc, g), rx = lf_rcp(pc.ipxx, g), ry = lf_rcp(pc.ipyy, g), rz = lf_rcp(pc.ipzz, g);
+  const double dt = I.dtime;
+  PartConst pc;
+  a.get_const(pc);
+  const LfRcp rv = lf_rcp(I.visc, g);
   auto spin_rate = [&](const double t[3], const double o[3], double k[3]) {
-    k[0] = lf_div(t[0] + o[1] * o[2] * (pc.ipyy - pc.ipzz), rx, g);
-    k[1] = lf_div(t[1] + o[2] * o[0] * (pc.ipzz - pc.ipxx), ry, g);
-    k[2] = lf_div(t[2] + o[0] * o[1] * (pc.ipxx - pc.ipyy), rz, g);
+    k[0] = lf_div(t[0] + o[1] * o[2] * (pc.ipyy - pc.ipzz), pc.ipxx, g);
+    k[1] = lf_div(t[1] + o[2] * o[0] * (pc.ipzz - pc.ipxx), pc.ipyy, g);
+    k[2] = lf_div(t[2] + o[0] * o[1] * (pc.ipxx - pc.ipyy), pc.ipzz, g);
   };
   auto at_wall = [&](double x, double y, double z, const Quat& q) {
-    double wn[3], arm[3], dx;
-    bool isect;
-    return wall_test(I.lx, pc, rmax, x, y, z, q, wn, arm, dx, isect) != 0 || isect;
+    if (off_wall(I.lx, fmax(pc.a, pc.b), x)) return false;
+    PartConst c;
+    a.get_const(c);
+    const Quat qq = q;
+    return wall_hit(I.lx, &c, x, y, z, &qq);
   };
-  double f[3], t[3], k1u[3], k1o[3], u1[3], o1[3], r[9];
-  Quat q1 = Q;
-  rotmat(Q, r);
-  {
-    SlipFast s;
-    fw_slip(pc, rv, U, uf, r, s, g);
-    fw_force(pc, s, r, f, g);
-    fw_torque(pc, rv, s, wv, O, r, t, g);
-  }
-  k1u[0] = f[0]; k1u[1] = f[1]; k1u[2] = f[2] + I.gravity;
-  spin_rate(t, O, k1o);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    u1[i] = U[i] + dt * k1u[i];
-    o1[i] = O[i] + dt * k1o[i];
-  }
-  fw_quaternion(q1, r, o1, dt, g);
-  if (at_wall(X[0] + dt * U[0], X[1] + dt * U[1], X[2] + dt * U[2], q1)) return false;
+  double f[3], t[3], r[9], k1[3];
+  Quat q1 = a.quat();
   rotmat(q1, r);
   {
     SlipFast s;
-    fw_slip(pc, rv, u1, uf, r, s, g);
+    double u[3], uf[3];
+    a.get3(kSlotU, u);
+    a.get3(kSlotFluid, uf);
+    fw_slip(pc, rv, u, uf, r, s, g);
     fw_force(pc, s, r, f, g);
-    fw_slip(pc, rv, U, uf, r, s, g);
+    f[2] = f[2] + I.gravity;
+    a.put3(kSlotWork, f);
+    double wv[3], o[3];
+    a.get3(kSlotFluid + 3, wv);
+    a.get3(kSlotO, o);
+    fw_torque(pc, rv, s, wv, o, r, t, g);
+    spin_rate(t, o, k1);
+    a.put3(kSlotWork + 3, k1);
+  }
+  // the predictor's velocity and spin, formed again where they are needed
+  auto predicted = [&](int col, int rate, double v[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) v[i] = a.get(col + i) + dt * a.get(rate + i);
+  };
+  double o1[3];
+  predicted(kSlotO, kSlotWork + 3, o1);
+  fw_quaternion(q1, r, o1, dt, g);
+  if (at_wall(a.get(0) + dt * a.get(3), a.get(1) + dt * a.get(4), a.get(2) + dt * a.get(5), q1)) return false;
+  a.put_quat(q1);
+  rotmat(q1, r);
+  {
+    SlipFast s;
+    double u[3], uf[3];
+    predicted(kSlotU, kSlotWork, u);
+    a.get3(kSlotFluid, uf);
+    fw_slip(pc, rv, u, uf, r, s, g);
+    fw_force(pc, s, r, f, g);
+  }
+  {
+    SlipFast s;
+    double u[3], uf[3], wv[3];
+    a.get3(kSlotU, u);
+    a.get3(kSlotFluid, uf);
+    fw_slip(pc, rv, u, uf, r, s, g);
+    a.get3(kSlotFluid + 3, wv);
+    predicted(kSlotO, kSlotWork + 3, o1);
     fw_torque(pc, rv, s, wv, o1, r, t, g);
   }
   double k2o[3];
   spin_rate(t, o1, k2o);
   const double k2u[3] = {f[0], f[1], f[2] + I.gravity};
-  double xn[3], un[3], on[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    xn[i] = X[i] + 0.5 * dt * (U[i] + u1[i]);
-    un[i] = U[i] + 0.5 * dt * (k1u[i] + k2u[i]);
-    on[i] = O[i] + 0.5 * dt * (k1o[i] + k2o[i]);
+    const double u = a.get(kSlotU + i), k1u = a.get(kSlotWork + i);
+    xn[i] = a.get(i) + 0.5 * dt * (u + (u + dt * k1u));
+    un[i] = u + 0.5 * dt * (k1u + k2u[i]);
+    on[i] = a.get(kSlotO + i) + 0.5 * dt * (a.get(kSlotWork + 3 + i) + k2o[i]);
   }
-  if (at_wall(xn[0], xn[1], xn[2], q1)) return false;
-  fw_quaternion(q1, r, on, dt, g);
-  if (!g.ok()) return false;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) { X[i] = xn[i]; U[i] = un[i]; O[i] = on[i]; }
-  Q = q1;
-  return true;
+  qn = a.quat();
+  if (at_wall(xn[0], xn[1], xn[2], qn)) return false;
+  fw_quaternion(qn, r, on, dt, g);
+  return g.ok();
 }
 
 }  // namespace gp
