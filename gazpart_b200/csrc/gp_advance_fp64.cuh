@@ -194,7 +194,7 @@ GP_LF void fw_sincos(double x, double& s, double& c, LfGuard& g) {
 // slip64 with what the correlations take of it.
 struct SlipFast {
   bool moving;   // the slip is not zero (a particle set off with the fluid's velocity)
-  double p[3], umag, syz, sphi, cphi;
+  double p[3], umag, syz, rep, phi, sphi, cphi;
   Log2 lrep, lsin, lcos;
 };
 GP_LF void fw_slip(const PartConst& pc, const LfRcp& rv, const double u[3], const double uf[3], const double r[9],
@@ -203,12 +203,13 @@ GP_LF void fw_slip(const PartConst& pc, const LfRcp& rv, const double u[3], cons
   const double pp = p[0] * p[0] + p[1] * p[1] + p[2] * p[2];
   s.moving = pp != 0.0;
   if (!s.moving) return;
-  const double rep = lf_quot(lf_sqrt(pp, g) * pc.deq, rv);
+  s.rep = lf_quot(lf_sqrt(pp, g) * pc.deq, rv);
   matvec_t(r, p, s.p);
   s.syz = lf_sqrt(s.p[1] * s.p[1] + s.p[2] * s.p[2], g);
   s.umag = lf_sqrt(s.p[0] * s.p[0] + s.p[1] * s.p[1] + s.p[2] * s.p[2], g);
-  fw_sincos(fabs(atan(lf_div(s.syz, s.p[0], g))), s.sphi, s.cphi, g);
-  s.lrep = fw_log2(rep, g, -200, 20);
+  s.phi = fabs(atan(lf_div(s.syz, s.p[0], g)));
+  fw_sincos(s.phi, s.sphi, s.cphi, g);
+  s.lrep = fw_log2(s.rep, g, -200, 20);
   s.lsin = fw_log2(s.sphi, g, -60, 1);
   s.lcos = fw_log2(s.cphi, g, -60, 1);
 }

@@ -1268,7 +1268,7 @@ int gp_stat_partfluid(gp_ctx *c, int32_t ig, double *out) {
   const int slot = ig - 1;
   size_groups(c, slot);
   const int ng = c->group_n[slot];
-  constexpr int kBlocks = 148 * 3;
+  constexpr int kBlocks = 148 * 10;   // resident
   if (!c->d_stat_partial) {
     GP_TRY(dalloc(&c->d_stat_partial, (size_t)kBlocks * kStatMaxGroups * kNStatPartfluid));
     GP_TRY(dalloc(&c->d_stat_out, (size_t)kStatMaxGroups * kNStatPartfluid));
