@@ -978,6 +978,22 @@ int gp_set_field_slot(gp_ctx *c, int32_t field, int32_t comp, const double *src,
   return GP_OK;
 }
 
+}  // extern "C"
+
+namespace gp {
+
+int couple_field(gp_ctx *c, int32_t field, const double *vel, const double *vort) {
+  const gp_ctx::FieldSlot &f = c->fields[field];
+  launch_field_nodes(f.ptr, c->prm.precision, f.nx, f.ny, f.nz, vel, vort, c->stream);
+  GP_CK(cudaGetLastError());
+  GP_CK(cudaStreamSynchronize(c->stream));
+  return GP_OK;
+}
+
+}  // namespace gp
+
+extern "C" {
+
 int gp_set_field(gp_ctx *c, int32_t comp, const double *src, int32_t src_layout, int32_t ghost_mode,
                  int32_t on_device) {
   return gp_set_field_slot(c, 0, comp, src, src_layout, ghost_mode, on_device);

@@ -9,9 +9,9 @@
 //   5. û = û_{n+1}^* + dt/2 RHS2; PROJ_DIVFREE; û *= FILTER        (:145-170, proj_divfree.f90)
 //   6. u = IFFT(û)                                                (:178-187)
 // The transforms are cuFFT's (D2Z forward, Z2D backward, both unnormalised as P3DFFT's
-// are), the three components of a vector field in one batched call; every step between
-// them is one element-wise kernel per stage, in FP64 and without FMA contraction, in the
-// reference's evaluation order.  A step makes 7 batched calls (21 transforms).  Wavenumbers follow
+// are), the three components of a vector field in one batched call; what lies between two
+// of them is one element-wise kernel (five a step), in FP64 and without FMA contraction, in
+// the reference's evaluation order.  A step makes 7 batched calls (21 transforms).  Wavenumbers follow
 // meshing.f90:96-140 (KX = (I-1) KFIRST on the half-spectrum, KY and KZ signed), and the
 // aliasing filter meshing.f90:144-180 (sharp or smooth, RTRUNC), computed per mode.
 // The stochastic forcing of STEADY runs (ADV_FORCING, ADD_FORCING3) is not part of it.
@@ -21,6 +21,7 @@
 #include <cmath>
 
 #include "../../include/gazpart_gpu.h"
+#include "gp_launch.h"
 #include "gp_types.h"
 
 struct gp_dns {
@@ -34,7 +35,7 @@ struct gp_dns {
   // [3][z][y][x/2+1]
   double *u = nullptr;            // velocity
   double *t = nullptr;            // vorticity, then u x ω
-  cufftDoubleComplex *uh = nullptr, *unp1 = nullptr, *w = nullptr, *tmp = nullptr;
+  cufftDoubleComplex *uh = nullptr, *unp1 = nullptr, *w = nullptr;
   size_t np = 0, nh = 0;          // points of one component
 };
 
@@ -55,8 +56,11 @@ struct Spec {
   double kfirst;
 };
 
+// 32-bit divisions: 2^32 modes of one component are more than the GPU's memory.
 __device__ __forceinline__ void wavenumbers(const Spec &s, int64_t e, double &kx, double &ky, double &kz) {
-  const int i = (int)(e % s.nxh), j = (int)((e / s.nxh) % s.ny), k = (int)(e / ((int64_t)s.nxh * s.ny));
+  const unsigned row = (unsigned)e / (unsigned)s.nxh;
+  const int i = (int)((unsigned)e - row * (unsigned)s.nxh), k = (int)(row / (unsigned)s.ny);
+  const int j = (int)(row - (unsigned)k * (unsigned)s.ny);
   kx = (double)i * s.kfirst;                                     // (I-1)*KFIRST
   ky = (j + 1 <= s.ny / 2 + 1) ? (double)j * s.kfirst : (double)(j - s.ny) * s.kfirst;
   kz = (k + 1 <= s.nz / 2 + 1) ? (double)k * s.kfirst : (double)(k - s.nz) * s.kfirst;
@@ -67,22 +71,40 @@ __device__ __forceinline__ cufftDoubleComplex cmul_i_real(cufftDoubleComplex a, 
   return make_cuDoubleComplex(-a.y * r, a.x * r);
 }
 
-// VORTX..Z = i k x û (nonlinear_terms.f90:81-92); the outputs are copies the backward
-// transform may overwrite.
-__global__ void k_vorticity_hat(Spec s, const cufftDoubleComplex *__restrict__ in, cufftDoubleComplex *out) {
+__device__ __forceinline__ cufftDoubleComplex scale(cufftDoubleComplex a, double r) {
+  return make_cuDoubleComplex(a.x * r, a.y * r);
+}
+__device__ __forceinline__ cufftDoubleComplex add(cufftDoubleComplex a, cufftDoubleComplex b) {
+  return make_cuDoubleComplex(a.x + b.x, a.y + b.y);
+}
+__device__ __forceinline__ cufftDoubleComplex sub(cufftDoubleComplex a, cufftDoubleComplex b) {
+  return make_cuDoubleComplex(a.x - b.x, a.y - b.y);
+}
+
+// VORTX..Z = i k x û (nonlinear_terms.f90:81-92)
+__device__ __forceinline__ void curl_hat(double kx, double ky, double kz, const cufftDoubleComplex u[3],
+                                         cufftDoubleComplex o[3]) {
+  const cufftDoubleComplex a = cmul_i_real(u[2], ky), b = cmul_i_real(u[1], kz);
+  const cufftDoubleComplex c = cmul_i_real(u[0], kz), d = cmul_i_real(u[2], kx);
+  const cufftDoubleComplex f = cmul_i_real(u[1], kx), g = cmul_i_real(u[0], ky);
+  o[0] = make_cuDoubleComplex(a.x - b.x, a.y - b.y);
+  o[1] = make_cuDoubleComplex(c.x - d.x, c.y - d.y);
+  o[2] = make_cuDoubleComplex(f.x - g.x, f.y - g.y);
+}
+
+// The vorticity's modes from the transformed velocity, which is scaled by FACTOR here (it
+// may be the same array).
+__global__ void k_vorticity_hat(Spec s, double factor, const cufftDoubleComplex *in, cufftDoubleComplex *out) {
   const int64_t n = (int64_t)s.nxh * s.ny * s.nz;
-  const cufftDoubleComplex *uh = in, *vh = in + n, *wh = in + 2 * n;
-  cufftDoubleComplex *ox = out, *oy = out + n, *oz = out + 2 * n;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     double kx, ky, kz;
     wavenumbers(s, e, kx, ky, kz);
-    const cufftDoubleComplex U = uh[e], V = vh[e], W = wh[e];
-    const cufftDoubleComplex a = cmul_i_real(W, ky), b = cmul_i_real(V, kz);
-    const cufftDoubleComplex c = cmul_i_real(U, kz), d = cmul_i_real(W, kx);
-    const cufftDoubleComplex f = cmul_i_real(V, kx), g = cmul_i_real(U, ky);
-    ox[e] = make_cuDoubleComplex(a.x - b.x, a.y - b.y);
-    oy[e] = make_cuDoubleComplex(c.x - d.x, c.y - d.y);
-    oz[e] = make_cuDoubleComplex(f.x - g.x, f.y - g.y);
+    const cufftDoubleComplex u[3] = {scale(in[e], factor), scale(in[n + e], factor), scale(in[2 * n + e], factor)};
+    cufftDoubleComplex o[3];
+    curl_hat(kx, ky, kz, u, o);
+    out[e] = o[0];
+    out[n + e] = o[1];
+    out[2 * n + e] = o[2];
   }
 }
 
@@ -96,16 +118,6 @@ __global__ void k_cross(int64_t n, const double *__restrict__ vel, double *z) {
     zy[e] = w[e] * a - u[e] * c;
     zz[e] = u[e] * b - v[e] * a;
   }
-}
-
-__device__ __forceinline__ cufftDoubleComplex scale(cufftDoubleComplex a, double r) {
-  return make_cuDoubleComplex(a.x * r, a.y * r);
-}
-__device__ __forceinline__ cufftDoubleComplex add(cufftDoubleComplex a, cufftDoubleComplex b) {
-  return make_cuDoubleComplex(a.x + b.x, a.y + b.y);
-}
-__device__ __forceinline__ cufftDoubleComplex sub(cufftDoubleComplex a, cufftDoubleComplex b) {
-  return make_cuDoubleComplex(a.x - b.x, a.y - b.y);
 }
 
 // The projected nonlinear term of nonlinear_terms.f90:119-160 from the transformed
@@ -124,28 +136,32 @@ __device__ __forceinline__ void rhs_of(double kx, double ky, double kz, double f
   r[2] = add(sub(sub(zero, scale(tx, kz * kx / k2)), scale(ty, kz * ky / k2)), scale(tz, (kx * kx + ky * ky) / k2));
 }
 
-// adv_fluid.f90:95-110: the first stage with the integrating factor.
-__global__ void k_stage1(Spec s, double factor, double visc, double dtime, cufftDoubleComplex *hat,
-                         cufftDoubleComplex *np1, const cufftDoubleComplex *__restrict__ t3) {
+// adv_fluid.f90:95-110: the first stage with the integrating factor.  hat holds the
+// transformed velocity, not yet scaled, and receives the predictor; t3 the transformed
+// u x ζ, and receives the predictor's vorticity: both go straight into the backward
+// transforms, which may overwrite them.  Bound by memory (128^3: 255 MB in 48 us); apart, the
+// stage took 37, and the scaling, the predictor's copy for the transform and the vorticity,
+// one pass over its arrays each, 14 to 20 more.
+__global__ void k_stage1(Spec s, double factor, double visc, double dtime, cufftDoubleComplex *__restrict__ hat,
+                         cufftDoubleComplex *__restrict__ np1, cufftDoubleComplex *__restrict__ t3) {
   const int64_t n = (int64_t)s.nxh * s.ny * s.nz;
-  cufftDoubleComplex *uh = hat, *vh = hat + n, *wh = hat + 2 * n;
-  cufftDoubleComplex *unp1 = np1, *vnp1 = np1 + n, *wnp1 = np1 + 2 * n;
-  const cufftDoubleComplex *tx = t3, *ty = t3 + n, *tz = t3 + 2 * n;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     double kx, ky, kz;
     wavenumbers(s, e, kx, ky, kz);
-    cufftDoubleComplex r[3];
-    rhs_of(kx, ky, kz, factor, tx[e], ty[e], tz[e], r);
+    cufftDoubleComplex r[3], u[3];
+    rhs_of(kx, ky, kz, factor, t3[e], t3[n + e], t3[2 * n + e], r);
     const double kappa2 = kx * kx + ky * ky + kz * kz;
     const double ef = exp(-visc * kappa2 * dtime);
-    cufftDoubleComplex *out_np1[3] = {unp1, vnp1, wnp1};
-    cufftDoubleComplex *io[3] = {uh, vh, wh};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const cufftDoubleComplex a = io[c][e];
-      out_np1[c][e] = scale(add(a, scale(r[c], dtime / 2)), ef);
-      io[c][e] = scale(add(a, scale(r[c], dtime)), ef);
+      const cufftDoubleComplex a = scale(hat[c * n + e], factor);
+      np1[c * n + e] = scale(add(a, scale(r[c], dtime / 2)), ef);
+      u[c] = scale(add(a, scale(r[c], dtime)), ef);
+      hat[c * n + e] = u[c];
     }
+    curl_hat(kx, ky, kz, u, r);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) t3[c * n + e] = r[c];
   }
 }
 
@@ -192,17 +208,11 @@ __global__ void k_stage2(Spec s, double factor, double dtime, double klast, int 
   }
 }
 
-__global__ void k_scale_spec(int64_t n, double factor, cufftDoubleComplex *a) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
-    a[e] = scale(a[e], factor);
-}
-
 int grid_of(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 148 * 16); }
 
-// NONLINEAR_TERMS: leaves FFT(u x ζ) (unscaled) in d->w.
-int nonlinear(gp_dns *d, const Spec &s) {
-  const int64_t nh = (int64_t)d->nh, np = (int64_t)d->np;
-  k_vorticity_hat<<<grid_of(nh), 256, 0, d->stream>>>(s, d->uh, d->w);
+// NONLINEAR_TERMS from the vorticity's modes in d->w: leaves FFT(u x ζ) (unscaled) there.
+int nonlinear(gp_dns *d) {
+  const int64_t np = (int64_t)d->np;
   if (cufftExecZ2D(d->bwd, d->w, d->t) != CUFFT_SUCCESS) return GP_ECUDA;
   k_cross<<<grid_of(np), 256, 0, d->stream>>>(np, d->u, d->t);
   if (cufftExecD2Z(d->fwd, d->t, d->w) != CUFFT_SUCCESS) return GP_ECUDA;
@@ -244,7 +254,6 @@ int gp_dns_create(const gp_params *p, int32_t aliascontrol, double rtrunc, gp_dn
   if (!rc) rc = alloc(&d->uh, 3 * d->nh);
   if (!rc) rc = alloc(&d->unp1, 3 * d->nh);
   if (!rc) rc = alloc(&d->w, 3 * d->nh);
-  if (!rc) rc = alloc(&d->tmp, 3 * d->nh);
   if (!rc) {
     long long dims[3] = {d->nz, d->ny, d->nx};
     size_t ws = 0;
@@ -278,7 +287,7 @@ int gp_dns_destroy(gp_dns *d) {
     cufftDestroy(d->fwd);
     cufftDestroy(d->bwd);
   }
-  cudaFree(d->u); cudaFree(d->t); cudaFree(d->uh); cudaFree(d->unp1); cudaFree(d->w); cudaFree(d->tmp);
+  cudaFree(d->u); cudaFree(d->t); cudaFree(d->uh); cudaFree(d->unp1); cudaFree(d->w);
   if (d->stream) cudaStreamDestroy(d->stream);
   delete d;
   return GP_OK;
@@ -308,22 +317,17 @@ int gp_adv_fluid(gp_dns *d, int32_t /*ncycle*/) {
   using namespace gp;
   if (!d) return GP_EBADARG;
   const Spec s = {d->nxh, d->ny, d->nz, d->kfirst};
-  const int64_t n3 = 3 * (int64_t)d->nh;
   const int g = grid_of((int64_t)d->nh);
-  // 1. û = FFT(u) * FACTOR (the forward transform leaves u as it is)
+  // 1. û = FFT(u) (the forward transform leaves u as it is); FACTOR comes with each use
   if (cufftExecD2Z(d->fwd, d->u, d->uh) != CUFFT_SUCCESS) return GP_ECUDA;
-  k_scale_spec<<<grid_of(n3), 256, 0, d->stream>>>(n3, d->factor, d->uh);
   // 2-3. first stage
-  int rc = nonlinear(d, s);
+  k_vorticity_hat<<<g, 256, 0, d->stream>>>(s, d->factor, d->uh, d->w);
+  int rc = nonlinear(d);
   if (rc) return rc;
   k_stage1<<<g, 256, 0, d->stream>>>(s, d->factor, d->visc, d->dtime, d->uh, d->unp1, d->w);
-  // 4. the predictor in physical space (from a copy: the backward transform overwrites
-  //    its input, and û is still needed), then the second nonlinear term
-  if (cudaMemcpyAsync(d->tmp, d->uh, n3 * sizeof(cufftDoubleComplex), cudaMemcpyDeviceToDevice, d->stream) !=
-      cudaSuccess)
-    return GP_ECUDA;
-  if (cufftExecZ2D(d->bwd, d->tmp, d->u) != CUFFT_SUCCESS) return GP_ECUDA;
-  rc = nonlinear(d, s);
+  // 4. the predictor in physical space, then the second nonlinear term
+  if (cufftExecZ2D(d->bwd, d->uh, d->u) != CUFFT_SUCCESS) return GP_ECUDA;
+  rc = nonlinear(d);
   if (rc) return rc;
   // 5. corrector, projection, filter
   k_stage2<<<g, 256, 0, d->stream>>>(s, d->factor, d->dtime, d->klast, d->aliascontrol, d->rtrunc,
@@ -338,11 +342,9 @@ int gp_adv_fluid(gp_dns *d, int32_t /*ncycle*/) {
 static int vorticity_to_t(gp_dns *d) {
   using namespace gp;
   const Spec s = {d->nxh, d->ny, d->nz, d->kfirst};
-  const int64_t n3 = 3 * (int64_t)d->nh;
   if (cufftExecD2Z(d->fwd, d->u, d->w) != CUFFT_SUCCESS) return GP_ECUDA;
-  k_scale_spec<<<grid_of(n3), 256, 0, d->stream>>>(n3, d->factor, d->w);
-  k_vorticity_hat<<<grid_of((int64_t)d->nh), 256, 0, d->stream>>>(s, d->w, d->unp1);
-  if (cufftExecZ2D(d->bwd, d->unp1, d->t) != CUFFT_SUCCESS) return GP_ECUDA;
+  k_vorticity_hat<<<grid_of((int64_t)d->nh), 256, 0, d->stream>>>(s, d->factor, d->w, d->w);
+  if (cufftExecZ2D(d->bwd, d->w, d->t) != CUFFT_SUCCESS) return GP_ECUDA;
   return cudaGetLastError() == cudaSuccess ? GP_OK : GP_ECUDA;
 }
 
@@ -364,21 +366,14 @@ int gp_dns_couple(gp_dns *d, gp_ctx *ctx, int32_t field, int32_t with_vorticity)
   const int rs = gp_field_shape(ctx, field, dims);
   if (rs) return rs;
   if (dims[0] != d->nx || dims[1] != d->ny || dims[2] != d->nz) return GP_EBADARG;   // other meshes
-  if (cudaStreamSynchronize(d->stream) != cudaSuccess) return GP_ECUDA;
-  // FLUIDCOMM (main.f90:499-505): the velocity's y and z ghosts are periodic copies
-  for (int c = 0; c < 3; ++c) {
-    const int rc = gp_set_field_slot(ctx, field, c, d->u + c * d->np, GP_LAYOUT_INTERIOR, GP_GHOST_PERIODIC, 1);
-    if (rc) return rc;
-  }
   if (with_vorticity) {
-    // vorticity of the current field, with zero ghosts as the reference's arrays have
-    int rc = vorticity_to_t(d);
-    if (!rc && cudaStreamSynchronize(d->stream) != cudaSuccess) rc = GP_ECUDA;
-    for (int c = 0; c < 3 && !rc; ++c)
-      rc = gp_set_field_slot(ctx, field, 3 + c, d->t + c * d->np, GP_LAYOUT_INTERIOR, GP_GHOST_ZERO, 1);
+    const int rc = vorticity_to_t(d);
     if (rc) return rc;
   }
-  return GP_OK;
+  if (cudaStreamSynchronize(d->stream) != cudaSuccess) return GP_ECUDA;
+  // FLUIDCOMM (main.f90:499-505): the velocity's y and z ghosts are periodic copies; the
+  // vorticity's are zero, as the reference's arrays have them
+  return gp::couple_field(ctx, field, d->u, with_vorticity ? d->t : nullptr);
 }
 
 }  // extern "C"

@@ -129,6 +129,12 @@ void launch_search(const InstDev *insts, const PoolView *pv, int64_t n, SearchAr
                    int64_t cap_pairs, Status *st, int grid, cudaStream_t s);
 void launch_match(const CollRec *coll, const unsigned long long *ncoll, int64_t cap_coll, unsigned long long *best1,
                   int8_t *matched, int8_t *state, Status *st, cudaStream_t s);
+// All nodes of an internal field from interior arrays, three components back to back each:
+// the velocity with periodic ghosts and, unless null, the vorticity with zero ghosts.
+void launch_field_nodes(void *dst, int prec, int nx, int ny, int nz, const double *vel, const double *vort,
+                        cudaStream_t s);
+// The same into a context's field slot (of the same mesh); returns when it is done.
+int couple_field(gp_ctx *c, int32_t field, const double *vel, const double *vort);
 void launch_field_layout(void *dst, int prec, int nx, int ny, int nz, int ncomp, int comp, const double *src,
                          int src_layout, int ghost_mode, cudaStream_t s);
 void launch_retire(const PoolView *pv, int64_t n, int inst, cudaStream_t s);
