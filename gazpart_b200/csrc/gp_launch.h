@@ -138,8 +138,14 @@ int couple_field(gp_ctx *c, int32_t field, const double *vel, const double *vort
 void launch_field_layout(void *dst, int prec, int nx, int ny, int nz, int ncomp, int comp, const double *src,
                          int src_layout, int ghost_mode, cudaStream_t s);
 void launch_retire(const PoolView *pv, int64_t n, int inst, cudaStream_t s);
-void launch_init_pool(const PoolView *pv, int64_t begin, int64_t n, int inst, const double *cols,
-                      const double *pcs, int64_t ld, int64_t src, cudaStream_t s);
+// One particle's constants, as an argument.
+struct ConstRow {
+  double v[kNConst];
+};
+// Particles of one class into pool slots [begin, begin + n) from columns of leading dimension
+// ld, from row src on; pcs null: all have the constants `row`.
+void launch_init_pool(const PoolView *pv, int64_t begin, int64_t n, int inst, const double *cols, const double *pcs,
+                      const ConstRow &row, int64_t ld, int64_t src, cudaStream_t s);
 void launch_connectivity(int nxb, int nyb, int nzb, int periodicity, int32_t *ncon, int32_t *con, cudaStream_t s);
 
 // --- gp_state.cu: the state columns between the caller's order and the pool's ---

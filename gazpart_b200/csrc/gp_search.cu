@@ -839,24 +839,24 @@ void launch_retire(const PoolView *pv, int64_t n, int inst, cudaStream_t s) {
 // One class into pool slots [begin, begin+n): particle k of the class is column entry
 // src + k of the staged arrays (leading dimension ld); ids are 0-based within the class.
 __global__ void k_init_pool(const PoolView *__restrict__ pv, int64_t begin, int64_t n, int inst,
-                            const double *__restrict__ cols, const double *__restrict__ pcs, int64_t ld,
-                            int64_t src) {
+                            const double *__restrict__ cols, const double *__restrict__ pcs, ConstRow row,
+                            int64_t ld, int64_t src) {
   const PoolView P = *pv;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = begin + k, e = src + k;
 #pragma unroll
     for (int c = 0; c < kNState; ++c) P.st[c][i] = cols[c * ld + e];
 #pragma unroll
-    for (int c = 0; c < kNConst; ++c) P.pc[c][i] = pcs[c * ld + e];
+    for (int c = 0; c < kNConst; ++c) P.pc[c][i] = pcs ? pcs[c * ld + e] : row.v[c];
     P.id[i] = (int32_t)k;
     P.inst[i] = inst;
   }
 }
 
 void launch_init_pool(const PoolView *pv, int64_t begin, int64_t n, int inst, const double *cols, const double *pcs,
-                      int64_t ld, int64_t src, cudaStream_t s) {
+                      const ConstRow &row, int64_t ld, int64_t src, cudaStream_t s) {
   if (n <= 0) return;
-  k_init_pool<<<148 * 8, 256, 0, s>>>(pv, begin, n, inst, cols, pcs, ld, src);
+  k_init_pool<<<148 * 8, 256, 0, s>>>(pv, begin, n, inst, cols, pcs, row, ld, src);
 }
 
 __global__ void k_iota(int32_t *a, int64_t n) {
