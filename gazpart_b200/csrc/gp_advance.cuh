@@ -814,13 +814,14 @@ __device__ __forceinline__ void gather_warp_fp64(const InstDev* __restrict__ ins
 // runs of 4 (48 by single lanes).
 inline int gather_run(int64_t n) {
   constexpr int64_t kWarps = 148 * 16;   // resident
-  return n > 16 * kWarps ? 32 : (n > 8 * kWarps ? 16 : (n > 4 * kWarps ? 8 : 4));
+  return n > kOrderedMin ? kOrderedRun : (n > 8 * kWarps ? 16 : (n > 4 * kWarps ? 8 : 4));
 }
 
 template <bool kMixed>
 __global__ void __launch_bounds__(256, GP_GATHER_MIN_BLOCKS) k_gather(const InstDev* __restrict__ insts,
                                                 const PoolView* __restrict__ src_pv,
                                                 const int32_t* __restrict__ perm, int64_t n, int run,
+                                                const int32_t* __restrict__ order,
                                                 double* const* __restrict__ fluid,
                                                 unsigned long long* __restrict__ ticket, Status* st) {
   __shared__ double results[kMixed ? 1 : 8 * 6 * 32];   // one 6 x 32 block a warp (FP64 form)
@@ -829,8 +830,9 @@ __global__ void __launch_bounds__(256, GP_GATHER_MIN_BLOCKS) k_gather(const Inst
   for (;;) {
     unsigned long long wt = 0;
     if (lane == 0) wt = atomicAdd(ticket, 1ull);
-    const int64_t w = (int64_t)__shfl_sync(0xffffffffu, wt, 0);
+    int64_t w = (int64_t)__shfl_sync(0xffffffffu, wt, 0);
     if (w * run >= n) break;
+    if (order != nullptr) w = order[w];
     const int64_t j = w * run + lane;
     const bool own = lane < run && j < n;
     int inst = -1;

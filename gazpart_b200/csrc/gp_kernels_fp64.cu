@@ -18,11 +18,12 @@ template __global__ void k_integrate_fix<false>(const InstDev *, const PoolView 
                                                 uint32_t *, PoolView *, PoolView *, unsigned long long *,
                                                 unsigned long long *, Status *);
 template __global__ void k_gather<false>(const InstDev *, const PoolView *, const int32_t *, int64_t, int,
-                                         double *const *, unsigned long long *, Status *);
+                                         const int32_t *, double *const *, unsigned long long *, Status *);
 
 void launch_gather_fp64(const InstDev *insts, const PoolView *pv, const int32_t *perm, int64_t n,
-                      double *const *fluid, unsigned long long *ticket, Status *st, int grid, cudaStream_t s) {
-  k_gather<false><<<grid, 256, 0, s>>>(insts, pv, perm, n, gather_run(n), fluid, ticket, st);
+                      const int32_t *order, double *const *fluid, unsigned long long *ticket, Status *st, int grid, cudaStream_t s) {
+  k_gather<false><<<grid, 256, 0, s>>>(insts, pv, perm, n, order ? kOrderedRun : gather_run(n), order, fluid,
+                                                   ticket, st);
 }
 
 void launch_integrate_fp64(const InstDev *insts, PoolView *pv, PoolView *pv_alt, const int32_t *perm, int64_t n,

@@ -15,8 +15,10 @@ struct TailRec;   // gp_contact.cuh
 // the two views (so *pv is current afterwards) and takes the gather's ticket back to zero.
 // With mark non-null, the speculative pass: marked particles are left to
 // launch_integrate_fix_*, which does both.  done: a counter, zero between launches.
+// order (may be null): the order in which the gather takes runs of kOrderedRun slots
+// (launch_run_order).
 void launch_gather_fp64(const InstDev *insts, const PoolView *pv, const int32_t *perm, int64_t n,
-                      double *const *fluid, unsigned long long *ticket, Status *st, int grid, cudaStream_t s);
+                      const int32_t *order, double *const *fluid, unsigned long long *ticket, Status *st, int grid, cudaStream_t s);
 void launch_integrate_fp64(const InstDev *insts, PoolView *pv, PoolView *pv_alt, const int32_t *perm, int64_t n,
                          double *const *fluid, Status *st, int grid, unsigned long long *done,
                          unsigned long long *ticket, cudaStream_t s, uint32_t *mark = nullptr);
@@ -95,7 +97,7 @@ void launch_collision_stats(const CollRec *coll, const unsigned long long *ncoll
 
 // --- gp_kernels_mixed.cu ---
 void launch_gather_mixed(const InstDev *insts, const PoolView *pv, const int32_t *perm, int64_t n,
-                      double *const *fluid, unsigned long long *ticket, Status *st, int grid, cudaStream_t s);
+                      const int32_t *order, double *const *fluid, unsigned long long *ticket, Status *st, int grid, cudaStream_t s);
 void launch_integrate_mixed(const InstDev *insts, PoolView *pv, PoolView *pv_alt, const int32_t *perm, int64_t n,
                          double *const *fluid, Status *st, int grid, unsigned long long *done,
                          unsigned long long *ticket, cudaStream_t s, uint32_t *mark = nullptr);
@@ -146,6 +148,9 @@ struct ConstRow {
 // ld, from row src on; pcs null: all have the constants `row`.
 void launch_init_pool(const PoolView *pv, int64_t begin, int64_t n, int inst, const double *cols, const double *pcs,
                       const ConstRow &row, int64_t ld, int64_t src, cudaStream_t s);
+// A permutation of the runs of kOrderedRun slots in [0, n), the classes' (instances with
+// begin and count set) interleaved by the fraction of the class that lies before them.
+void launch_run_order(const InstDev *insts, int ninst, int64_t n, int32_t *order, cudaStream_t s);
 void launch_connectivity(int nxb, int nyb, int nzb, int periodicity, int32_t *ncon, int32_t *con, cudaStream_t s);
 
 // --- gp_state.cu: the state columns between the caller's order and the pool's ---

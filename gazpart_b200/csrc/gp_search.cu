@@ -868,6 +868,42 @@ void launch_iota(int32_t *a, int64_t n, cudaStream_t s) {
   if (n > 0) k_iota<<<148 * 8, 256, 0, s>>>(a, n);
 }
 
+// The slots are in class order and, within a class, in cell order, so classes on one field
+// each sweep the whole of it, one after the other, and read it from HBM again.  Taken by the
+// fraction of its class that lies before it, a run's neighbours in time are the other
+// classes' runs at the same height, and the field passes through the L2 once.
+// Run t belongs to the class of its middle slot m (or, the last one, of the last slot); runs
+// are ordered by ((m - begin) / count, class), and a run's place is the number of runs of
+// each class before it.
+__global__ void k_run_order(const InstDev *__restrict__ insts, int ninst, int64_t n, int32_t *__restrict__ order) {
+  const int64_t nruns = (n + kOrderedRun - 1) / kOrderedRun;
+  constexpr int64_t kMid = kOrderedRun / 2;
+  // first run whose middle is at slot x or later
+  auto run_from = [&](int64_t x) { return min((x + kOrderedRun - 1 - kMid) / kOrderedRun, nruns); };
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nruns; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t m = t * kOrderedRun + kMid, slot = min(m, n - 1);
+    int own = 0;
+    while (own < ninst - 1 && !(slot < insts[own].begin + insts[own].count)) ++own;
+    const int64_t mine = insts[own].count, f = m - insts[own].begin;
+    int64_t place = 0;
+    for (int k = 0; k < ninst; ++k) {
+      const int64_t b = insts[k].begin, cnt = insts[k].count;
+      if (cnt == 0) continue;
+      // the last run's middle may lie past the last class
+      const int64_t first = run_from(b), end = b + cnt == n ? nruns : run_from(b + cnt);
+      // middles m' of class k with (m' - b) / cnt before f / mine: m' - b < x
+      const int64_t v = f * cnt, q = v / mine;
+      const int64_t x = (k < own || v % mine != 0) ? q + 1 : q;
+      place += k == own ? t - first : min(max(run_from(b + x), first), end) - first;
+    }
+    order[place] = (int32_t)t;
+  }
+}
+
+void launch_run_order(const InstDev *insts, int ninst, int64_t n, int32_t *order, cudaStream_t s) {
+  if (n > 0) k_run_order<<<148 * 4, 128, 0, s>>>(insts, ninst, n, order);
+}
+
 // COLLISION_BOX_CONNECTIVITY (collision_box_connectivity.f90:42-322), NPROC=1.
 __global__ void k_connectivity(int NXB, int NYB, int NZB, int periodicity, int32_t *ncon, int32_t *con) {
   const int64_t nbox = (int64_t)NXB * NYB * NZB;

@@ -85,6 +85,8 @@ struct PairRec {
   unsigned long long k2;            // (id_home << 34) | (slot << 30) | id_near
 };
 constexpr int64_t kMaxInstanceParticles = (int64_t)1 << 30;
+constexpr int kOrderedRun = 32;     // slots a gather's warp takes at a time ...
+constexpr int64_t kOrderedMin = 16 * 148 * 16;   // ... for more than 16 for each resident warp
 constexpr int kMaxClasses = 1024;   // classes (instances) per context
 
 // A colliding pair with what COLLISION_RESPONSE needs.
