@@ -357,10 +357,13 @@ __device__ __forceinline__ PairEnd pair_end(const PoolView &P, int32_t i) {
 // One candidate (sorted positions s, qs) of the sweep that passed near_float: FP64
 // bounding-sphere test, centre-line separation test, reference box adjacency, then emission
 // with the reference's ordering keys.
-__device__ __forceinline__ void search_candidate(const InstDev *__restrict__ insts, const PoolView &P,
-                                                 const SearchArrays &sa, int32_t s, int32_t qs, PairRec *pairs,
-                                                 unsigned long long *npairs, int64_t cap, Status *st) {
-  const int32_t pslot = sa.sorted[s], qslot = sa.sorted[qs];
+// Out of line, so that its FP64 state takes no registers from the sweep.
+static __device__ __noinline__ void search_candidate(const InstDev *__restrict__ insts, const PoolView *pv,
+                                                     const int32_t *sorted, uint32_t *mark, int32_t s, int32_t qs,
+                                                     PairRec *pairs, unsigned long long *npairs, int64_t cap,
+                                                     Status *st) {
+  const PoolView &P = *pv;
+  const int32_t pslot = sorted[s], qslot = sorted[qs];
   const InstDev &I = insts[P.inst[pslot]];
   const bool perx = I.periodicity != 0;
   const PairEnd p = pair_end(P, pslot), q = pair_end(P, qslot);
@@ -417,7 +420,7 @@ __device__ __forceinline__ void search_candidate(const InstDev *__restrict__ ins
   r.near = home_is_p ? qslot : pslot;
   r.k1 = ijk;
   r.k2 = ((unsigned long long)idh << 34) | ((unsigned long long)slot << 30) | (unsigned long long)idn;
-  emit_pair(pairs, npairs, cap, r, sa.mark, st);
+  emit_pair(pairs, npairs, cap, r, mark, st);
 }
 
 __device__ __forceinline__ int wrap_cell(int c, int n) { return c < 0 ? c + n : (c >= n ? c - n : c); }
@@ -435,20 +438,27 @@ __device__ __forceinline__ int wrap_cell(int c, int n) { return c < 0 ? c + n : 
 #define GP_SEARCH_MIN_BLOCKS 4
 #endif
 
-constexpr int kSearchThreads = 256;
+constexpr int kSearchThreads = 288;
 constexpr int kMaxRanges = 10;   // 5 rows, each at most two contiguous ranges
 
 // Each lane takes one home particle (32 consecutive sorted particles per warp) and works
 // out the ranges of sorted particles its half stencil must test: the five forward rows
-// of cells, trimmed to the cells within reach.  The warp then tests all its homes'
+// of cells, trimmed to the cells within reach; the rows' cell records are requested in two
+// batches, each before the first of them is looked at.  The warp then tests all its homes'
 // candidates together, 32 at a time: candidate idx of the warp's concatenated lists goes
 // to lane idx mod 32, which looks up the owning home and range in shared memory.  Lanes
-// stay busy however unevenly the candidates fall among the homes.  Homes above the cut
+// stay busy however unevenly the candidates fall among the homes.  The candidates that pass
+// wait in the warp's queue until there are 32 for the exact tests, or the warp has no more
+// homes: one at a time in their lanes they held up the whole warp, once for 32 homes at
+// 16.8 M particles and seven times in a packed ensemble.  Homes above the cut
 // radius sweep their wide stencil afterwards, each on its own lane.  Everything up to the
 // candidates that pass is FP32, widened by the slack that covers its rounding; about one
-// candidate in 500 passes and reads its two particles from the pool.  What bounds it is
-// instruction issue and the latency of the cell lookups.  Measured (B200): 16.8 M particles
-// 1.84 ms with FP64 home records in sorted columns -> 1.52, 1 M 0.105 -> 0.078.
+// candidate in 100 passes and reads its two particles from the pool.  What bounds it is the
+// latency of the lookups, half of it in forming the ranges, with 36 warps an SM (1.28 ms at
+// 16.8 M particles with 32, 1.24 with 40: what then spills goes through an L1 that the lookups
+// fill; 1.23 with one batch).
+// Measured (B200): 16.8 M particles 1.55 ms -> 1.20, 1 M 0.080 -> 0.069, 20,000 packed 0.041
+// -> 0.031.
 __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search(
     const InstDev *__restrict__ insts, const PoolView *__restrict__ pv, int64_t n, SearchArrays sa,
     PairRec *__restrict__ pairs, unsigned long long *npairs, int64_t cap, Status *st) {
@@ -461,9 +471,13 @@ __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search
   __shared__ int32_t rstart[kSearchThreads][kMaxRanges];   // first sorted particle of a range
   __shared__ int32_t rcum[kSearchThreads][kMaxRanges];     // candidates of the home before it
   __shared__ int8_t rnum[kSearchThreads];
+  __shared__ int2 passed[kSearchThreads / 32][64];  // candidates for the exact tests
   constexpr unsigned kFull = 0xffffffffu;
   const PoolView &P = *pv;
   const int t = threadIdx.x, lane = t & 31, wbase = t & ~31;
+  const unsigned before = (1u << lane) - 1u;
+  int2 *queue = passed[t >> 5];
+  int nq = 0;
   const int64_t nact = sa.cell_start[sa.ncells];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s0 = (int64_t)blockIdx.x * blockDim.x + wbase; s0 < nact; s0 += stride) {
@@ -482,6 +496,14 @@ __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search
         cell_coords(I, cell, cx, cy, cz);
         const int nfx = I.nfx, nfy = I.nfy, nfz = I.nfz;
         const bool perx = I.periodicity != 0;
+        const int xl = cx > 0 ? cx - 1 : nfx - 1, xr = cx + 1 < nfx ? cx + 1 : 0;
+        const int yu = wrap_cell(cy + 1, nfy), zu = wrap_cell(cz + 1, nfz);
+        const int32_t rows[5] = {cell_row(I, cy, cz), cell_row(I, yu, cz), cell_row(I, wrap_cell(cy - 1, nfy), zu),
+                                 cell_row(I, cy, zu), cell_row(I, yu, zu)};
+        // the row's three cells: where the left begins, the middle begins and ends, the right
+        // ends, and the largest radius in each
+        int32_t sl[5], sm[5], se[5], sr[5];
+        float ml[5], mm[5], mr[5];
         // Small candidates have radius <= rcut, so only cells whose box comes within
         // R = rp + rcut of this particle can hold a partner: rows and end cells farther
         // away are skipped (distances to the neighbour boxes from the offsets inside the
@@ -502,43 +524,44 @@ __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search
             ++nr;
           }
         };
-        for (int r = 0; r < 5; ++r) {
-          int ry = cy, rz = cz;
-          float dyz2 = 0.f;
-          if (r == 1) {
-            ry = wrap_cell(cy + 1, nfy);
-            dyz2 = dyh * dyh;
-          } else if (r > 1) {
-            rz = wrap_cell(cz + 1, nfz);
-            ry = wrap_cell(cy + (r - 3), nfy);
-            const float dyb = (r == 2) ? dyl : (r == 4 ? dyh : 0.f);
-            dyz2 = dyb * dyb + dzh * dzh;
+        auto request = [&](int r) {
+          const int32_t row = rows[r];
+          sl[r] = sm[r] = 0;
+          ml[r] = mm[r] = 0.f;
+          if (r > 0) {   // the home's own row begins at the home
+            sl[r] = __ldg(sa.cell_start + row + xl);
+            sm[r] = __ldg(sa.cell_start + row + cx);
+            ml[r] = __ldg(sa.cell_rmax + row + xl);
+            mm[r] = __ldg(sa.cell_rmax + row + cx);
           }
-          if (dyz2 > R2) continue;
-          const int32_t row = cell_row(I, ry, rz);
+          se[r] = __ldg(sa.cell_start + row + cx + 1);
+          sr[r] = __ldg(sa.cell_start + row + xr + 1);
+          mr[r] = __ldg(sa.cell_rmax + row + xr);
+        };
+        request(0); request(1);
+#pragma unroll
+        for (int r = 0; r < 5; ++r) {
+          if (r == 2) { request(2); request(3); request(4); }
+          const float dyb = r == 2 ? dyl : (r == 3 ? 0.f : dyh);
+          const float dyz2 = r == 0 ? 0.f : (r == 1 ? dyh * dyh : dyb * dyb + dzh * dzh);
           // each cell within reach of its own largest radius
-          auto reaches = [&](int32_t k, float d2) {
-            const float m = rp + sa.cell_rmax[k];
+          auto reaches = [&](float most, float d2) {
+            const float m = rp + most;
             return d2 <= R2 && d2 <= m * m;
           };
-          const int32_t cl = row + (cx > 0 ? cx - 1 : nfx - 1), cm = row + cx;
-          const int32_t cr = row + (cx + 1 < nfx ? cx + 1 : 0);
-          const bool use_l = r > 0 && left_ok && reaches(cl, dxl * dxl + dyz2);
-          const bool use_r = right_ok && reaches(cr, dxh * dxh + dyz2);
+          const bool row_ok = dyz2 <= R2;
+          const bool use_l = r > 0 && row_ok && left_ok && reaches(ml[r], dxl * dxl + dyz2);
+          const bool use_r = row_ok && right_ok && reaches(mr[r], dxh * dxh + dyz2);
           // the home cell from s+1 on; its neighbours' middle cell whenever an end is used
-          const bool use_m = r == 0 || use_l || use_r || reaches(cm, dyz2);
-          int32_t a0 = 0, a1 = 0;
-          if (use_m) {
-            a0 = r == 0 ? (int32_t)s + 1 : sa.cell_start[cm];
-            a1 = sa.cell_start[cm + 1];
-          }
-          if (use_l) {
-            const int32_t b0 = sa.cell_start[cl];
-            if (cl + 1 == cm) a0 = b0; else add(b0, sa.cell_start[cl + 1]);
-          }
-          if (use_r) {
-            const int32_t b1 = sa.cell_start[cr + 1];
-            if (cr == cm + 1) a1 = b1; else add(sa.cell_start[cr], b1);
+          const bool use_m = r == 0 || use_l || use_r || (row_ok && reaches(mm[r], dyz2));
+          int32_t a0 = r == 0 ? (int32_t)s + 1 : sm[r], a1 = use_m ? se[r] : a0;
+          if (use_l && cx > 0) a0 = sl[r];
+          if (use_r && cx + 1 < nfx) a1 = sr[r];
+          if ((use_l && cx == 0) || (use_r && cx + 1 == nfx)) {   // nfx >= 3: one of the two
+            const int32_t row = rows[r];
+            const int32_t b0 = use_l && cx == 0 ? sl[r] : __ldg(sa.cell_start + row);
+            const int32_t b1 = use_l && cx == 0 ? __ldg(sa.cell_start + row + nfx) : sr[r];
+            add(b0, b1);
           }
           add(a0, a1);
         }
@@ -565,15 +588,28 @@ __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search
         if (o + step < 32 && e <= idx) o += step;
       }
       const int32_t eo = __shfl_sync(kFull, excl, o);
+      bool pass = false;
+      int32_t q = 0;
       if (idx < total) {
         const int to = wbase + o;
         const int32_t k = idx - eo;
         int j = 0;
         const int no = rnum[to];
         while (j + 1 < no && rcum[to][j + 1] <= k) ++j;
-        const int32_t q = rstart[to][j] + (k - rcum[to][j]);
-        if (near_float<false>(sa.spk[q], q, 0, homesf[to]))
-          search_candidate(insts, P, sa, (int32_t)(s0 + o), q, pairs, npairs, cap, st);
+        q = rstart[to][j] + (k - rcum[to][j]);
+        pass = near_float<false>(sa.spk[q], q, 0, homesf[to]);
+      }
+      const unsigned m = __ballot_sync(kFull, pass);
+      if (m != 0u) {
+        if (pass) queue[nq + __popc(m & before)] = make_int2((int32_t)(s0 + o), q);
+        nq += __popc(m);
+        __syncwarp();
+        if (nq >= 32) {
+          nq -= 32;
+          const int2 e = queue[nq + lane];
+          search_candidate(insts, &P, sa.sorted, sa.mark, e.x, e.y, pairs, npairs, cap, st);
+          __syncwarp();
+        }
       }
     }
     if (large) {
@@ -601,7 +637,7 @@ __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search
             const int32_t q1 = sa.cell_start[row + w + len];
             for (int32_t qs = sa.cell_start[row + w]; qs < q1; ++qs)
               if (qs != s && near_float<true>(sa.spk[qs], qs, (int32_t)s, hf))
-                search_candidate(insts, P, sa, (int32_t)s, qs, pairs, npairs, cap, st);
+                search_candidate(insts, &P, sa.sorted, sa.mark, (int32_t)s, qs, pairs, npairs, cap, st);
             x += len;
           }
         }
@@ -609,11 +645,12 @@ __global__ void __launch_bounds__(kSearchThreads, GP_SEARCH_MIN_BLOCKS) k_search
     }
     __syncwarp();   // the records are rewritten by the warp's next 32 homes
   }
+  if (lane < nq) search_candidate(insts, &P, sa.sorted, sa.mark, queue[lane].x, queue[lane].y, pairs, npairs, cap, st);
 }
 
 void launch_search(const InstDev *insts, const PoolView *pv, int64_t n, SearchArrays sa, PairRec *pairs, unsigned long long *npairs,
                    int64_t cap_pairs, Status *st, int grid, cudaStream_t s) {
-  k_search<<<grid, 256, 0, s>>>(insts, pv, n, sa, pairs, npairs, cap_pairs, st);
+  k_search<<<grid, kSearchThreads, 0, s>>>(insts, pv, n, sa, pairs, npairs, cap_pairs, st);
 }
 
 // ---------------------------------------------------------------------------
