@@ -374,7 +374,7 @@ static __device__ __forceinline__ int wall_rebound(double ecw, double muw, const
 }
 
 // collision_response.f90:1-437 (inertia of particle 1 for both bodies, :140-145).
-static __device__ __noinline__ int collision_response(double ecp, double mup, double ipxx, double ipyy, double ipzz,
+static __device__ __forceinline__ int collision_response(double ecp, double mup, double ipxx, double ipyy, double ipzz,
                                          double u1[3], double o1[3], const Quat& q1,
                                          double u2[3], double o2[3], const Quat& q2,
                                          const double r1[3], const double r2[3], const double n[3]) {
