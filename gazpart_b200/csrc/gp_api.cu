@@ -160,8 +160,10 @@ struct gp_ctx {
   std::map<std::pair<int, int>, ClassProps> classes;
   // captured multi-step graphs, by step count
   std::map<int, cudaGraphExec_t> graphs;
-  // launch grids (blocks), GP_TUNE_* order; gp_autotune picks them on the live workload
-  int tune[GP_NTUNE] = {148 * 8, 148 * 4, 148 * 4, 148 * 4};
+  // launch grids (blocks), GP_TUNE_* order; gp_autotune picks them on the live workload.  The
+  // gather's warps take their work from a counter; 16 blocks per SM cost a step of 1 M 7 us
+  // more than 4.
+  int tune[GP_NTUNE] = {148 * 4, 148 * 4, 148 * 8, 148 * 4};
   // gather of step s+1 on the side stream, overlapping step s's contact solves (multi-step
   // graphs).  The solves end one by one and leave SMs idle, so it pays at every size: ms a
   // step of five-step graphs without / with it (B200), FP64 10,000 particles 0.173 / 0.160,
