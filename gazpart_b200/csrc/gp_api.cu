@@ -166,9 +166,9 @@ struct gp_ctx {
   int tune[GP_NTUNE] = {148 * 4, 148 * 4, 148 * 8, 148 * 4};
   // gather of step s+1 on the side stream, overlapping step s's contact solves (multi-step
   // graphs).  The solves end one by one and leave SMs idle, so it pays at every size: ms a
-  // step of five-step graphs without / with it (B200), FP64 10,000 particles 0.173 / 0.160,
-  // 20,000 packed 0.389 / 0.372, 1 M 1.158 / 1.012, 4 M 3.98 / 3.74; mixed 100,000 0.265 /
-  // 0.245, 1 M 0.850 / 0.750, 16.8 M 8.81 / 8.54, 24 classes of 2 M in all 1.366 / 1.269.
+  // step of five-step graphs without / with it (B200), FP64 10,000 particles 0.160 / 0.148,
+  // 20,000 packed 0.377 / 0.363, 1 M 1.115 / 0.977, 4 M 3.81 / 3.60; mixed 100,000 0.251 /
+  // 0.228, 1 M 0.807 / 0.706, 16.8 M 7.81 / 7.54, 24 classes of 2 M in all 0.967 / 0.883.
   // The autotuner times both, and the speculative integrate too.
   bool overlap = true;
   // with the overlap, step s+1's integrate also runs on the side stream, speculatively,
@@ -865,6 +865,7 @@ int gp_ctx_create(const gp_params *params, gp_ctx **out) {
   }
   if (!rc) rc = dalloc(&c->d_status, 1);
   if (!rc && cudaMemset(c->d_status, 0, sizeof(Status)) != cudaSuccess) rc = GP_ECUDA;
+  if (!rc && cudaStreamSynchronize(nullptr) != cudaSuccess) rc = GP_ECUDA;   // as in gp_add_field
   if (!rc) rc = upload_inst(c);
   if (!rc && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = GP_ECUDA;
   if (!rc) {
@@ -1011,7 +1012,12 @@ int gp_add_field(gp_ctx *c, int32_t nx, int32_t ny, int32_t nz, double lx, doubl
   const size_t bytes = (size_t)(nx + 3) * (ny + 4) * (nz + 4) * kFieldStride * elem;
   void *ptr = nullptr;
   if (cudaMalloc(&ptr, bytes) != cudaSuccess) return GP_ENOMEM;
-  if (cudaMemset(ptr, 0, bytes) != cudaSuccess) { cudaFree(ptr); return GP_ECUDA; }
+  // the fill is over before the field is written: c->stream does not wait for the default
+  // stream, on which cudaMemset leaves it
+  if (cudaMemset(ptr, 0, bytes) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) {
+    cudaFree(ptr);
+    return GP_ECUDA;
+  }
   c->fields.push_back({ptr, nx, ny, nz, lx, ly, lz});
   *field = (int32_t)c->fields.size() - 1;
   return GP_OK;
@@ -1410,8 +1416,9 @@ int gp_collision_stats_enable(gp_ctx *c, int32_t on) {
     c->cap_cst = 0;
     if (!c->d_colacc) {
       GP_TRY(dalloc(&c->d_colacc, (size_t)kMaxClasses * kStatMaxGroups * kStatMaxGroups * kNStatCollision));
-      GP_CK(cudaMemset(c->d_colacc, 0,
-                       (size_t)kMaxClasses * kStatMaxGroups * kStatMaxGroups * kNStatCollision * sizeof(double)));
+      GP_CK(cudaMemsetAsync(c->d_colacc, 0,
+                            (size_t)kMaxClasses * kStatMaxGroups * kStatMaxGroups * kNStatCollision * sizeof(double),
+                            c->stream));
     }
     // every candidate pair may be in contact
     GP_TRY(dalloc(&c->d_cst, (size_t)std::max<int64_t>(c->cap_pairs, 1)));
