@@ -74,7 +74,8 @@ __device__ __forceinline__ void cell_coords(const InstDev &I, int32_t cell, int 
 }
 
 // Of the `grid` blocks that fill the chip (eight per SM: the binning waits for its scattered
-// accesses, 16.8 M particles 0.65 ms with four, 0.58 with eight) only those that get a
+// accesses, 16.8 M particles 0.65 ms with four; 0.58 with eight, half of the scatter's then
+// waiting for the others' registers, 0.52 with all of them resident) only those that get a
 // particle: 10,000 particles 19 us with eight per SM, 17 so.
 constexpr int kBinThreads = 256;
 static int bin_blocks(int64_t n, int grid) {
@@ -240,10 +241,10 @@ __device__ __forceinline__ bool in_boxes(double v, double vmin, double edge, int
 // is judged by goes into sorted order (20 bytes a particle); the few candidates that pass
 // read the pool.  What bounds it is the scattered traffic: with sixteen sorted columns
 // (112 bytes written, 100 read) and three arrays of cells cleared by themselves the whole
-// binning took 1.07 ms at 16.8 M particles, with these two 0.58 (B200).  Numbering the
+// binning took 1.07 ms at 16.8 M particles, with these two 0.52 (B200).  Numbering the
 // cells in bricks of 4 x 4 x 8, 4 x 4 x 4 or 2 x 2 x 8 for the gather's sake left the
 // gather as it was (3.22 ms each) and took 0.04 more in the search.
-__global__ void k_bin_scatter(const InstDev *__restrict__ insts, const PoolView *__restrict__ pv, int64_t n,
+__global__ void __launch_bounds__(kBinThreads, 8) k_bin_scatter(const InstDev *__restrict__ insts, const PoolView *__restrict__ pv, int64_t n,
                               SearchArrays sa, Status *st) {
   if (step_halted(st)) return;
   const PoolView P = *pv;
