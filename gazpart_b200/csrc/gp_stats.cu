@@ -255,7 +255,8 @@ __global__ void __launch_bounds__(32 * kStatWarps, 10)
         for (int r = 0; r < kStatSummed; ++r) t[r * kStatTile] = v[stat_of_row(r)];
       }
     }
-    unsigned todo = __ballot_sync(0xffffffffu, g >= 0);   // and the tile is complete
+    __syncwarp();   // the tile is complete: votes and shuffles order no memory accesses
+    unsigned todo = __ballot_sync(0xffffffffu, g >= 0);
     while (todo) {
       const int gg = __shfl_sync(0xffffffffu, g, __ffs(todo) - 1);
       const unsigned mine = __ballot_sync(0xffffffffu, g == gg);
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__(32 * kStatWarps, 10)
         acc[warp][gg][35] += m;
       }
     }
-    __syncwarp();
+    __syncwarp();   // and read, before the next one is written
   }
   __syncthreads();
   for (int t = threadIdx.x; t < ngroups * kNStatPartfluid; t += blockDim.x) {
