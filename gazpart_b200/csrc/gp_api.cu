@@ -597,8 +597,15 @@ int enqueue_integrate_fix(gp_ctx *c) {
 }
 
 int enqueue_advance(gp_ctx *c) {
+  // With retired particles among the slots the binning's order names slots beyond the n that
+  // the advance leaves; no binning need follow before the next advance, which then keeps
+  // the order that this one moves to.
+  const bool compacts = c->n_slots > c->n;
   GP_TRY(enqueue_gather(c, c->stream));
-  return enqueue_integrate(c);
+  GP_TRY(enqueue_integrate(c));
+  if (compacts) launch_iota(c->sa.sorted, c->n, c->stream);
+  GP_CK(cudaGetLastError());
+  return GP_OK;
 }
 
 // Binning of the search grid (also the cell order the next advance moves to).
