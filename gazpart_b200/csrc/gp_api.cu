@@ -267,19 +267,57 @@ StateCols cols_at(double *base, int64_t n) {
   return k;
 }
 
-// The caller's device columns, where the copy kernels may access them directly: memory of
-// this device, aligned.  False otherwise (then cudaMemcpy moves them, or reports why not).
-bool direct_cols(const gp_ctx *c, const double *const *cols, StateCols *out) {
+template <typename F>
+F driver_entry(const char *name) {
+  void *f = nullptr;
+  cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+  if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+    f = nullptr;
+  return reinterpret_cast<F>(f);
+}
+
+// Whether the `bytes` at p lie in p's allocation: 1 yes, 0 no, -1 not known (memory mapped
+// piece by piece, whose next piece may follow; no answer from the driver).
+int within_allocation(const void *p, size_t bytes) {
+  using Range = CUresult (*)(CUdeviceptr *, size_t *, CUdeviceptr);
+  using Retain = CUresult (*)(CUmemGenericAllocationHandle *, void *);
+  using Release = CUresult (*)(CUmemGenericAllocationHandle);
+  // looked up once (a thread-safe static initialisation)
+  static const Range range = driver_entry<Range>("cuMemGetAddressRange");
+  static const Retain retain = driver_entry<Retain>("cuMemRetainAllocationHandle");
+  static const Release release = driver_entry<Release>("cuMemRelease");
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+  if (!range || range(&base, &size, at) != CUDA_SUCCESS) return -1;
+  if (at - base <= size && bytes <= size - (at - base)) return 1;
+  CUmemGenericAllocationHandle h;
+  if (!retain || !release) return -1;
+  if (retain(&h, const_cast<void *>(p)) != CUDA_SUCCESS) return 0;
+  release(h);
+  return -1;
+}
+
+// The caller's device columns of n values, where the copy kernels may access them directly:
+// memory of this device, aligned, n values long.  *direct false otherwise (then cudaMemcpy
+// moves them, or reports why not); GP_EBADARG for a column that ends before its n values.
+// The extents cost a call 0.6 us (13 columns of 10,000 values in: 23.7 us -> 24.3).
+int direct_cols(const gp_ctx *c, const double *const *cols, int64_t n, StateCols *out, bool *direct) {
+  *direct = false;
   for (int i = 0; i < kNState; ++i) {
     cudaPointerAttributes a;
     if (!cols[i] || ((uintptr_t)cols[i] & 7u) || cudaPointerGetAttributes(&a, cols[i]) != cudaSuccess) {
       cudaGetLastError();
-      return false;
+      return GP_OK;
     }
-    if (a.type != cudaMemoryTypeDevice || a.device != c->device) return false;
+    if (a.type != cudaMemoryTypeDevice || a.device != c->device) return GP_OK;
+    const int in = within_allocation(cols[i], (size_t)n * sizeof(double));
+    if (in == 0) return GP_EBADARG;
+    if (in < 0) return GP_OK;
     out->p[i] = const_cast<double *>(cols[i]);
   }
-  return true;
+  *direct = true;
+  return GP_OK;
 }
 
 void read_state(gp_ctx *c, const StateCols &out, int64_t count, unsigned mask = kAllStateCols, int only = -1) {
@@ -1288,9 +1326,11 @@ int gp_add_class(gp_ctx *c, int32_t field, int64_t n, const double *const *cols,
 int gp_download_class(gp_ctx *c, int32_t ig, double *const *cols, int32_t on_device) {
   if (!c || !cols || ig < 1 || ig > (int)c->live.size() || !c->live[ig - 1]) return GP_EBADARG;
   const int64_t n = c->insts[ig - 1].count;
-  StateCols direct;
-  if (on_device && direct_cols(c, cols, &direct)) {
-    read_state(c, direct, n, kAllStateCols, ig - 1);
+  StateCols out;
+  bool direct = false;
+  if (on_device) GP_TRY(direct_cols(c, cols, n, &out, &direct));
+  if (direct) {
+    read_state(c, out, n, kAllStateCols, ig - 1);
     GP_CK(cudaGetLastError());
     GP_CK(cudaStreamSynchronize(c->stream));
     return GP_OK;
@@ -1477,9 +1517,11 @@ int gp_download_state(gp_ctx *c, int64_t n, double *const *cols, double *const *
   if (fluid && !c->prm.store_fluid) return GP_EBADARG;
   // the context's scratch buffer, kept between calls: a fresh allocation and its
   // release (which waits for the device) would cost more than the gather itself
-  StateCols direct;
-  if (on_device && !fluid && direct_cols(c, cols, &direct)) {
-    read_state(c, direct, n);
+  StateCols out;
+  bool direct = false;
+  if (on_device && !fluid) GP_TRY(direct_cols(c, cols, n, &out, &direct));
+  if (direct) {
+    read_state(c, out, n);
     GP_CK(cudaGetLastError());
     GP_CK(cudaStreamSynchronize(c->stream));
     return GP_OK;
@@ -1504,7 +1546,9 @@ int gp_download_state(gp_ctx *c, int64_t n, double *const *cols, double *const *
 int gp_put_state(gp_ctx *c, int64_t n, const double *const *cols, int32_t on_device) {
   if (!c || !cols || n != c->n) return GP_EBADARG;
   StateCols in;
-  if (!on_device || !direct_cols(c, cols, &in)) {
+  bool direct = false;
+  if (on_device) GP_TRY(direct_cols(c, cols, n, &in, &direct));
+  if (!direct) {
     GP_TRY(ensure_scratch(c, (size_t)kNState * n));
     for (int k = 0; k < kNState; ++k) GP_TRY(copy_in(c, c->d_scratch + (size_t)k * n, cols[k], n, on_device));
     in = cols_at(c->d_scratch, n);
