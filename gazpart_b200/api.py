@@ -304,6 +304,8 @@ class Context:
         keep, cols, dev = [], (C.c_void_p * 13)(), None
         for i, k in enumerate(STATE_KEYS):
             p, d, kk = _ptr(st[k])
+            if (kk.numel() if d else kk.size) < self.n:
+                raise ValueError(f"{k}: fewer than {self.n} values")
             cols[i] = p
             keep.append(kk)
             dev = d
@@ -329,6 +331,9 @@ class Context:
 
     def download_into(self, out: Dict[str, np.ndarray]) -> None:
         """Download the state columns into preallocated (e.g. pinned) float64 arrays."""
+        for k in STATE_KEYS:
+            if out[k].nbytes < 8 * self.n:
+                raise ValueError(f"{k}: no room for {self.n} float64 values")
         cols = (C.c_void_p * 13)(*[C.c_void_p(out[k].ctypes.data) for k in STATE_KEYS])
         check(_lib.lib().gp_download_state(self._h, self.n, cols, None, 0), "gp_download_state")
 
