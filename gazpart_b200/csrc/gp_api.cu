@@ -21,6 +21,7 @@
 
 #include "../../include/gazpart_gpu.h"
 #include "gp_launch.h"
+#include "gp_ticket.h"
 #include "gp_types.h"
 
 using namespace gp;
@@ -125,6 +126,7 @@ struct gp_ctx {
   int32_t *d_runs = nullptr;
   int64_t cap_runs = 0, runs_n = 0;
   const int32_t *run_order() const { return runs_n == n && n > 0 ? d_runs : nullptr; }
+  GatherTicket ticket;
   int64_t n_slots = 0;             // pool slots holding particles, retired ones included
   bool grid_ready = false;
   // pool
@@ -571,8 +573,23 @@ int ensure_field_map(gp_ctx *c) {
   return GP_OK;
 }
 
+int clear_ticket(gp_ctx *c, cudaStream_t s) {
+  GP_CK(cudaMemsetAsync(c->d_counters + 6, 0, sizeof(unsigned long long), s));
+  return GP_OK;
+}
+
+// Before a graph: one captured earlier has no clearing of its own, and a clearing captured
+// now would not run if the graph does not.
+int settle_ticket(gp_ctx *c) {
+  if (!c->ticket.stale()) return GP_OK;
+  GP_TRY(clear_ticket(c, c->stream));
+  c->ticket.paired();
+  return GP_OK;
+}
+
 // Stencil gather at x_n for the particles in the last binning's order, on stream s.
 int enqueue_gather(gp_ctx *c, cudaStream_t s) {
+  if (c->ticket.take()) GP_TRY(clear_ticket(c, s));
   GP_TRY(mark(c, 2 * GP_PHASE_GATHER, s));
   if (c->prm.precision == GP_PREC_MIXED && c->gather_staging == 1 && ensure_field_map(c) == GP_OK)
     // two blocks of four warps per SM are resident; the warps take their runs from the
@@ -598,6 +615,7 @@ int enqueue_integrate(gp_ctx *c) {
     launch_integrate_fp64(c->d_inst, c->d_pv, c->d_pv_alt, c->sa.sorted, c->n, c->d_fluid_cols, c->d_status,
                            c->tune[GP_TUNE_INTEGRATE], c->d_counters + 5, c->d_counters + 6, c->stream);
   GP_CK(cudaGetLastError());
+  c->ticket.paired();
   c->n_slots = c->n;   // the pass writes the active particles, in cell order, to slots [0, n)
   c->fluid_ok = true;  // and the fluid it used, at the same slots
   return mark(c, 2 * GP_PHASE_INTEGRATE + 1, c->stream);
@@ -629,6 +647,7 @@ int enqueue_integrate_fix(gp_ctx *c) {
                               c->d_fluid_cols, c->d_mark, c->d_status, 148 * 4, c->d_counters + 5, c->d_counters + 6,
                                c->stream);
   GP_CK(cudaGetLastError());
+  c->ticket.paired();
   c->n_slots = c->n;
   c->fluid_ok = true;
   return mark(c, 2 * GP_PHASE_INTEGRATE + 1, c->stream);
@@ -1671,6 +1690,7 @@ int capture_steps(gp_ctx *c, int nsteps, cudaEvent_t *marks, cudaGraph_t *g) {
 // Replays `nsteps` steps from the graph cache (one graph per step count in use; the
 // cache is bounded).
 int replay_steps(gp_ctx *c, int nsteps) {
+  GP_TRY(settle_ticket(c));
   auto it = c->graphs.find(nsteps);
   if (it == c->graphs.end()) {
     if (c->graphs.size() >= 8) drop_graph(c);
@@ -1709,6 +1729,7 @@ int gp_step(gp_ctx *c, int32_t nsteps) {
 
 int gp_step_timed(gp_ctx *c, int32_t nsteps, float *total_ms, float *phase_ms_avg, int32_t *kernels_per_step) {
   if (!c || c->n <= 0 || !c->grid_ready || nsteps <= 0) return GP_EBADARG;
+  GP_TRY(settle_ticket(c));
   // [0] start, then 2*GP_NPHASE per step (begin/end of each phase), then the end
   std::vector<cudaEvent_t> ev(2 + (size_t)nsteps * 2 * GP_NPHASE);
   for (auto &e : ev) GP_CK(cudaEventCreate(&e));
