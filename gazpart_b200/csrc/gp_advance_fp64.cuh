@@ -20,7 +20,11 @@
 // cosine 0.78 and 0.16 (CUDA's sincos 1.35 and 0.17); quotients and roots were equal to
 // CUDA's in every case.
 //
-// Measured (B200, integrate of one step): 1 M particles 0.58 -> 0.30 ms, 10,000 38 -> 21 us.
+// Exact zeros are inside the ranges: particles that settle in still fluid have them in the
+// spin and the torque at every step, bodies along or across the flow in the slip.
+//
+// Measured (B200, integrate of one step): 1 M particles 0.58 -> 0.30 ms, 10,000 38 -> 21 us;
+// 1 M settling in still fluid 0.61 -> 0.33 (1.17 where a zero raises the flag).
 #pragma once
 #include "gp_lm_fast.cuh"
 
@@ -191,10 +195,29 @@ GP_LF void fw_sincos(double x, double& s, double& c, LfGuard& g) {
   c = ((q + 1) & 2) ? -w : w;
 }
 
+// Quotients and roots that take an exact zero: in still fluid, or with a body along or across
+// the flow, components of the slip, the spin and the torque are zero at every step.
+// a / r.b for r.b > 0, the zero with a's sign (lf_quot's remainder would lose a negative one).
+// No guard: the caller knows that a is finite, or looks at what comes of it.
+GP_LF double fw_quot(double a, const LfRcp& r) {
+  const double q = __dmul_rn(a, r.y);
+  return __fma_rn(-__fma_rn(r.b, q, -a), r.y, q);
+}
+GP_LF bool is_zero(double a) { return (LfGuard::high(a) | __double2loint(a)) == 0; }
+GP_LF double fw_sqrt(double a, LfGuard& g) {
+  const bool zero = is_zero(a);
+  const double v = zero ? 1.0 : a;
+  g.in(v);
+  const double s = lf_root(v).b;
+  return zero ? 0.0 : s;
+}
+
 // slip64 with what the correlations take of it.
 struct SlipFast {
   bool moving;   // the slip is not zero (a particle set off with the fluid's velocity)
-  double p[3], umag, syz, rep, phi, sphi, cphi;
+  bool along;    // the slip is along the axis, its transverse parts are zero
+  double p[3], umag, rep, phi, sphi, cphi;
+  LfRcp syz;     // the transverse slip as a divisor (1 along the axis)
   Log2 lrep, lsin, lcos;
 };
 GP_LF void fw_slip(const PartConst& pc, const LfRcp& rv, const double u[3], const double uf[3], const double r[9],
@@ -205,12 +228,20 @@ GP_LF void fw_slip(const PartConst& pc, const LfRcp& rv, const double u[3], cons
   if (!s.moving) return;
   s.rep = lf_quot(lf_sqrt(pp, g) * pc.deq, rv);
   matvec_t(r, p, s.p);
-  s.syz = lf_sqrt(s.p[1] * s.p[1] + s.p[2] * s.p[2], g);
+  const double yz = s.p[1] * s.p[1] + s.p[2] * s.p[2];
+  s.along = is_zero(yz);
+  s.syz = lf_root(s.along ? 1.0 : yz);
+  g.in(s.along ? 1.0 : yz);
   s.umag = lf_sqrt(s.p[0] * s.p[0] + s.p[1] * s.p[1] + s.p[2] * s.p[2], g);
-  s.phi = fabs(atan(lf_div(s.syz, s.p[0], g)));
+  // across the axis the quotient is infinite, along it the sine is zero, and so is each of
+  // its powers (their exponents are above 1/2 from Re = 2^-100 on)
+  const bool across = is_zero(s.p[0]);
+  const double tphi = lf_quot(s.along ? 0.0 : s.syz.b, lf_rcp(across ? 1.0 : s.p[0], g));
+  s.phi = fabs(atan(across ? CUDART_INF : tphi));
   fw_sincos(s.phi, s.sphi, s.cphi, g);
-  s.lrep = fw_log2(s.rep, g, -200, 20);
-  s.lsin = fw_log2(s.sphi, g, -60, 1);
+  s.lrep = fw_log2(s.rep, g, s.along ? -100 : -200, 20);
+  s.lsin = fw_log2(s.along ? 1.0 : s.sphi, g, -160, 1);
+  if (s.along) s.lsin.hi = -4096.0;
   s.lcos = fw_log2(s.cphi, g, -60, 1);
 }
 
@@ -227,9 +258,8 @@ GP_LF void fw_force(const PartConst& pc, const SlipFast& s, const double r[9], d
   const double kd = pc.cdrag * cdrag * s.umag;
   double fd[3] = {kd * s.p[0], kd * s.p[1], kd * s.p[2]};
   const double kl = pc.cdrag * clift * (s.umag * s.umag);
-  const LfRcp ry = lf_rcp(s.syz, g);
-  double fl[3] = {kl * s.sphi * copysign(1.0, -s.p[0]), kl * s.cphi * lf_div(s.p[1], ry, g),
-                  kl * s.cphi * lf_div(s.p[2], ry, g)};
+  double fl[3] = {kl * s.sphi * copysign(1.0, -s.p[0]), kl * s.cphi * fw_quot(s.p[1], s.syz),
+                  kl * s.cphi * fw_quot(s.p[2], s.syz)};
   matvec(r, fd, fd);
   matvec(r, fl, fl);
 #pragma unroll
@@ -248,14 +278,13 @@ GP_LF void fw_torque(const PartConst& pc, const LfRcp& rv, const SlipFast& s, co
                        fw_pow(s.lsin, 0.116 + 0.748 * fw_pow(s.lrep, 0.041)) *
                        fw_pow(s.lcos, 0.221 + 0.657 * fw_pow(s.lrep, 0.044));
     const double cp = pc.cpitch * ctp * (s.umag * s.umag);
-    const LfRcp ry = lf_rcp(s.syz, g);
-    tp1 = cp * lf_div(fabs(s.p[2]), ry, g) * copysign(1.0, s.p[0] * s.p[2]);
-    tp2 = cp * lf_div(fabs(s.p[1]), ry, g) * copysign(1.0, s.p[0] * s.p[1]);
+    tp1 = cp * fw_quot(fabs(s.p[2]), s.syz) * copysign(1.0, s.p[0] * s.p[2]);
+    tp2 = cp * fw_quot(fabs(s.p[1]), s.syz) * copysign(1.0, s.p[0] * s.p[1]);
   }
   const double ww = o0 * o0 + o1 * o1 + o2 * o2;
   if (ww != 0.0) {
     const double rer = lf_quot(lf_sqrt(ww, g) * (pc.deq * pc.deq), rv);
-    const double oyz = lf_sqrt(o2 * o2 + o1 * o1, g);
+    const double oyz = fw_sqrt(o2 * o2 + o1 * o1, g);
     const Log2 l = fw_log2(rer, g, -300, 40);
     const double ctr = 0.573 * fw_pow(l, -0.154) + lf_quot(116.61, lf_rcp(rer, g));
     const double ctr2 = 1.244 * fw_pow(l, 0.239) + 378.12 * fw_pow(l, -0.789);
@@ -274,11 +303,11 @@ GP_LF void fw_quaternion(Quat& q, const double r[9], const double o[3], double d
   matvec(r, o, w);
   const double ww = w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
   if (ww == 0.0) return;
-  const double nrm = lf_sqrt(ww, g);
+  g.in(ww);
+  const LfRcp rn = lf_root(ww);
   double s, c;
-  fw_sincos((nrm * dt) / 2.0, s, c, g);
-  const LfRcp rn = lf_rcp(nrm, g);
-  const Quat map = {c, s * lf_div(w[0], rn, g), s * lf_div(w[1], rn, g), s * lf_div(w[2], rn, g)};
+  fw_sincos((rn.b * dt) / 2.0, s, c, g);
+  const Quat map = {c, s * fw_quot(w[0], rn), s * fw_quot(w[1], rn), s * fw_quot(w[2], rn)};
   q = mult_quat(map, q);
 }
 
@@ -336,9 +365,9 @@ GP_LF bool advance_particle_fast(const InstDev& I, const Slot& a, double xn[3], 
   a.get_const(pc);
   const LfRcp rv = lf_rcp(I.visc, g);
   auto spin_rate = [&](const double t[3], const double o[3], double k[3]) {
-    k[0] = lf_div(t[0] + o[1] * o[2] * (pc.ipyy - pc.ipzz), pc.ipxx, g);
-    k[1] = lf_div(t[1] + o[2] * o[0] * (pc.ipzz - pc.ipxx), pc.ipyy, g);
-    k[2] = lf_div(t[2] + o[0] * o[1] * (pc.ipxx - pc.ipyy), pc.ipzz, g);
+    k[0] = fw_quot(t[0] + o[1] * o[2] * (pc.ipyy - pc.ipzz), lf_rcp(pc.ipxx, g));
+    k[1] = fw_quot(t[1] + o[2] * o[0] * (pc.ipzz - pc.ipxx), lf_rcp(pc.ipyy, g));
+    k[2] = fw_quot(t[2] + o[0] * o[1] * (pc.ipxx - pc.ipyy), lf_rcp(pc.ipzz, g));
   };
   auto at_wall = [&](double x, double y, double z, const Quat& q) {
     if (off_wall(I.lx, fmax(pc.a, pc.b), x)) return false;
@@ -405,6 +434,8 @@ GP_LF bool advance_particle_fast(const InstDev& I, const Slot& a, double xn[3], 
     un[i] = u + 0.5 * dt * (k1u + k2u[i]);
     on[i] = a.get(kSlotO + i) + 0.5 * dt * (a.get(kSlotWork + 3 + i) + k2o[i]);
   }
+  // the spin's quotients are unguarded: both stages' end up here
+  g.finite(on[0]); g.finite(on[1]); g.finite(on[2]);
   qn = a.quat();
   if (at_wall(xn[0], xn[1], xn[2], qn)) return false;
   fw_quaternion(qn, r, on, dt, g);

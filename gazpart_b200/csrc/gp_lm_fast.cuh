@@ -45,6 +45,8 @@ struct LfGuard {
     const bool fine = (unsigned)(h - lo) < span || (h < lo && least > 0x3be6a1c6);   // the high word of rdwarf
     far = max(far, fine ? 0u : 0xffffffffu);
   }
+  // v is below 2^1023 in magnitude, neither infinite nor NaN
+  __device__ __forceinline__ void finite(double v) { far = max(far, high(v) < 0x7fe00000 ? 0u : 0xffffffffu); }
   static __device__ __forceinline__ int high(double v) { return __double2hiint(v) & 0x7fffffff; }
   __device__ __forceinline__ bool ok() const { return far < kSpan; }
 };

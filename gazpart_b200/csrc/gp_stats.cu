@@ -135,9 +135,8 @@ GP_LF bool partfluid_fast(const PartConst &pc, double rhof, double visc, double 
   rotmat(q, r);
   SlipFast s;
   fw_slip(pc, rv, U, uf, r, s, g);
-  if (!s.moving) return false;
+  if (!s.moving || s.along) return false;   // no guards there in the reference: NaN
   const double u2 = s.umag * s.umag;
-  const LfRcp ry = lf_rcp(s.syz, g);
   {
     const double cd0 = 18.12 * fw_pow(s.lrep, -1.023) + 4.26 * fw_pow(s.lrep, -0.384);
     const double cd90 = 21.52 * fw_pow(s.lrep, -0.990) + 2.86 * fw_pow(s.lrep, -0.260);
@@ -149,8 +148,8 @@ GP_LF bool partfluid_fast(const PartConst &pc, double rhof, double visc, double 
     double fd[3], fl[3];
     for (int k = 0; k < 3; ++k) fd[k] = kf * cdrag * s.umag * s.p[k];
     fl[0] = kf * clift * u2 * s.sphi * copysign(1.0, -s.p[0]);
-    fl[1] = kf * clift * u2 * s.cphi * lf_div(s.p[1], ry, g);
-    fl[2] = kf * clift * u2 * s.cphi * lf_div(s.p[2], ry, g);
+    fl[1] = kf * clift * u2 * s.cphi * fw_quot(s.p[1], s.syz);
+    fl[2] = kf * clift * u2 * s.cphi * fw_quot(s.p[2], s.syz);
     matvec(r, fd, fd);
     matvec(r, fl, fl);
     put(0, s.rep); put(1, cdrag); put(2, clift);
@@ -175,8 +174,8 @@ GP_LF bool partfluid_fast(const PartConst &pc, double rhof, double visc, double 
     const double ctr = 0.573 * fw_pow(l, -0.154) + lf_div(116.61, re_r, g);
     const double ctr2 = 1.244 * fw_pow(l, 0.239) + 378.12 * fw_pow(l, -0.789);
     const double kp = 0.25 * rp * 0.25 * ppi * (d2 * deq);
-    const double tp1 = kp * ctp * u2 * lf_div(fabs(s.p[2]), ry, g) * copysign(1.0, s.p[0] * s.p[2]);
-    const double tp2 = kp * ctp * u2 * lf_div(fabs(s.p[1]), ry, g) * copysign(1.0, s.p[0] * s.p[1]);
+    const double tp1 = kp * ctp * u2 * fw_quot(fabs(s.p[2]), s.syz) * copysign(1.0, s.p[0] * s.p[2]);
+    const double tp2 = kp * ctp * u2 * fw_quot(fabs(s.p[1]), s.syz) * copysign(1.0, s.p[0] * s.p[1]);
     const double h = deq / 2.0, h2 = h * h, h5 = h2 * h2 * h;
     const double tr0 = ctr * rp / 2.0 * h5 * fabs(o0) * o0;
     const double tr1 = ctr2 * rp / 2.0 * h5 * oyz * o1;
