@@ -164,15 +164,18 @@ GP_LF bool partfluid_fast(const PartConst &pc, double rhof, double visc, double 
     double curl[3];
     matvec_t(r, wv, curl);
     const double o0 = 0.5 * curl[0] - O[0], o1 = 0.5 * curl[1] - O[1], o2 = 0.5 * curl[2] - O[2];
-    const double omag = lf_sqrt(o0 * o0 + o1 * o1 + o2 * o2, g);
-    const double oyz = lf_sqrt(o2 * o2 + o1 * o1, g);
+    const double ww = o0 * o0 + o1 * o1 + o2 * o2;
+    const bool still = is_zero(ww);   // Re_r = 0, infinite coefficients as in the reference
+    const double omag = fw_sqrt(ww, g);
+    const double oyz = fw_sqrt(o2 * o2 + o1 * o1, g);
     const double re_r = lf_quot(omag * d2, rv);
     const double ctp = (0.935 * fw_pow(s.lrep, -0.146) + -0.469 * fw_pow(s.lrep, -0.145)) *
                        fw_pow(s.lsin, 0.116 + 0.748 * fw_pow(s.lrep, 0.041)) *
                        fw_pow(s.lcos, 0.221 + 0.657 * fw_pow(s.lrep, 0.044));
-    const Log2 l = fw_log2(re_r, g, -300, 40);
-    const double ctr = 0.573 * fw_pow(l, -0.154) + lf_div(116.61, re_r, g);
-    const double ctr2 = 1.244 * fw_pow(l, 0.239) + 378.12 * fw_pow(l, -0.789);
+    const double pole = still ? CUDART_INF : 0.0, re = still ? 1.0 : re_r;
+    const Log2 l = fw_log2(re, g, -300, 40);
+    const double ctr = 0.573 * fw_pow(l, -0.154) + lf_div(116.61, re, g) + pole;
+    const double ctr2 = 1.244 * fw_pow(l, 0.239) + 378.12 * fw_pow(l, -0.789) + pole;
     const double kp = 0.25 * rp * 0.25 * ppi * (d2 * deq);
     const double tp1 = kp * ctp * u2 * fw_quot(fabs(s.p[2]), s.syz) * copysign(1.0, s.p[0] * s.p[2]);
     const double tp2 = kp * ctp * u2 * fw_quot(fabs(s.p[1]), s.syz) * copysign(1.0, s.p[0] * s.p[1]);
@@ -184,7 +187,8 @@ GP_LF bool partfluid_fast(const PartConst &pc, double rhof, double visc, double 
     put(15, tp1); put(16, tp2);
     put(17, tr0); put(18, tr1); put(19, tr2);
     put(20, lf_sqrt(tp1 * tp1 + tp2 * tp2, g));
-    put(21, lf_sqrt(tr0 * tr0 + tr1 * tr1 + tr2 * tr2, g));
+    const double tt = tr0 * tr0 + tr1 * tr1 + tr2 * tr2;
+    put(21, still ? tt : lf_sqrt(still ? 1.0 : tt, g));   // still: infinite or NaN, its own root
   }
   // NaN for an oblate body, as in the reference
   double fbeta = apr == 1.0 ? 1.0 : CUDART_NAN;
