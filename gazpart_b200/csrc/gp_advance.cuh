@@ -945,7 +945,8 @@ GP_LF bool advance_mixed_slot(const InstDev& I, const Slot& a, const PoolView& S
   };
   predicted(kSlotO, kSlotConst + 3, o);
   quaternion_step_mixed<true>(q1, r, o[0], o[1], o[2], dt);
-  if (at_wall(a.get(0) + dt * a.get(3), a.get(1) + dt * a.get(4), a.get(2) + dt * a.get(5), q1)) return false;
+  if (at_wall(__fma_rn(dt, a.get(3), a.get(0)), __fma_rn(dt, a.get(4), a.get(1)), __fma_rn(dt, a.get(5), a.get(2)), q1))
+    return false;
   a.put_quat(q1);
   rotmat_f(q1, r);
   {
