@@ -20,12 +20,13 @@ from . import _lib
 from .api import PROP_KEYS, STATE_KEYS, Context, check
 
 # Device bytes one resident particle costs: two pool buffers (13 state + 10 constant
-# doubles, id, class), the six interpolated field values, 112 bytes for the search arrays
-# and the staging of its admission (cell, order, packed float4: 24; 13 state doubles while it
-# comes or goes), the matching words, its share of the pair and contact buffers, and the
-# contact queue's order (the particle's record of its last solves, a pair slot's order and
-# bin).
-BYTES_PER_PARTICLE = 2 * (23 * 8 + 8) + 6 * 8 + 112 + 17 + 24 + 26 + 4 + 5
+# doubles, id, class), the six interpolated field values, the search arrays (cell, order,
+# packed float4: 24; its share of the cells: 6), the 13 state doubles that stage it while it
+# comes or goes (an upper bound: the staging is as large as the largest job), the matching
+# words, its share of the pair and contact buffers, and the contact queue's order (the
+# particle's record of its last solves, a pair slot's order and bin).  Measured between 2^21 and
+# 2^22 particles: 643 each.  A job of many shapes takes 80 more a particle while its constants go in.
+BYTES_PER_PARTICLE = 2 * (23 * 8 + 8) + 6 * 8 + 24 + 6 + 13 * 8 + 17 + 24 + 28 + 4 + 5
 
 
 class GPJob(C.Structure):
