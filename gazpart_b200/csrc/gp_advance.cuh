@@ -1096,8 +1096,8 @@ __device__ __forceinline__ void finish_advance(PoolView* a, PoolView* b, unsigne
 //
 // What bounds it: 16 warps an SM, each in a chain of some 1,600 instructions; the step keeps
 // its state in shared memory (Slot) because the registers it spilled cost more than the
-// chain.  Measured (B200, one-step graphs): mixed 16.8 M particles 2.01 -> 1.59 ms (436
-// bytes a particle, 4.6 TB/s), 1 M 0.137 -> 0.117; FP64 1 M 0.298 -> 0.291.  Five and six
+// chain.  Measured (B200, one-step graphs): mixed 16.8 M particles 2.01 -> 1.59 ms (442
+// bytes a particle, 4.7 TB/s), 1 M 0.137 -> 0.117; FP64 1 M 0.298 -> 0.291.  Five and six
 // blocks per SM (96 and 80 registers): mixed 1.67 and 1.84, FP64 0.320 and 0.338.  Fetching a
 // particle's columns while the one before is advanced, with the state in registers, took
 // 2.11.

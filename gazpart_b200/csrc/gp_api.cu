@@ -1115,7 +1115,6 @@ InstDev class_template(const gp_ctx *c, int f) {
   return I;
 }
 
-// Host copy of the GP_NPROP property columns of n particles.
 // The property columns of n particles on the host: the caller's own arrays, or copies of
 // device ones in store.
 int read_props(gp_ctx *c, int64_t n, const double *const *props, int32_t on_device, std::vector<double> *store,
@@ -1172,9 +1171,6 @@ int class_setup(gp_ctx *c, const double *const *hp, int64_t off, int64_t cnt, do
   return setup_grids(I, max_emaj, rmax, rsmall, 0);
 }
 
-// After a change of the class table: caller-order offsets and search cells of the live
-// classes, the device table, the captured graphs, and (rebin) a binning pass so that
-// the next advance moves exactly the live particles.
 void size_groups(gp_ctx *c, int slot) {
   if ((int)c->group_dev.size() <= slot) {
     c->group_dev.resize(slot + 1, nullptr);
@@ -1217,6 +1213,9 @@ void order_runs(gp_ctx *c) {
   if (cudaGetLastError() == cudaSuccess) c->runs_n = c->n;
 }
 
+// After a change of the class table: caller-order offsets and search cells of the live
+// classes, the device table, the captured graphs, and (rebin) a binning pass so that
+// the next advance moves exactly the live particles.
 int refresh_classes(gp_ctx *c, bool rebin) {
   int64_t begin = 0, cells = 0;
   for (size_t k = 0; k < c->insts.size(); ++k) {

@@ -289,7 +289,6 @@ __global__ void k_response(const InstDev *__restrict__ insts, const PoolView *__
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&st->steps_done, 1ull);
   const PoolView P = *pv;
   const int64_t nc = (int64_t)min(*ncoll, (unsigned long long)cap_coll);
-  // neighbouring pairs go to different blocks
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nc; e += (int64_t)gridDim.x * blockDim.x) {
     if (state[e] != 1) continue;
     const CollRec r = coll[e];

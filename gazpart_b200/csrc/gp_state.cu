@@ -172,9 +172,9 @@ int grid_of(int64_t n) { return (int)min((n + kTile - 1) / kTile, (int64_t)148 *
 
 // From this many particles on the copy goes through rows.  All 13 columns, us a call with
 // its launch and wait (B200), column by column / through rows:
-//                   600,000       1 M        2 M        16.8 M
-//   into the pool    67 / 109   112 / 169   348 / 288   5183 / 2128
-//   out of it        74 / 106   257 / 164   873 / 281   9828 / 2060
+//                   600,000    800,000      1 M       1.6 M      1.8 M       2 M       16.8 M
+//   into the pool    59 / 98    81 / 130  108 / 157  216 / 232  261 / 254  327 / 279  5183 / 2128
+//   out of it        84 / 100  155 / 131  258 / 159  633 / 234  752 / 252  863 / 277  9828 / 2060
 // (13 staging copies and a column-by-column kernel before: 5780 and 10419 at 16.8 M, 82
 // and 74 at 10,000 where it now takes 28 and 23.)  Scattered writes leave the L2's reach
 // first.
