@@ -220,7 +220,7 @@ def gather_bytes_per_particle(components: int, field_bytes: int) -> int:
 # take consecutive runs of the cell order from one counter, so the figure does not
 # depend on the gather's grid.
 GATHER_TRAFFIC = {
-    ("c3_512cube_n16777216_fp32field", "mixed"): (286.2, "profiles/k_gather_k_integrate_c3_dram.md"),
+    ("c3_512cube_n16777216_fp32field", "mixed"): (285.4, "profiles/gather_integrate_512cube_n16777216_dram.md"),
 }
 
 
