@@ -171,7 +171,9 @@ int gp_set_field(gp_ctx *ctx, int32_t comp, const double *src, int32_t src_layou
                  int32_t ghost_mode, int32_t on_device);
 
 /* Particle state (PART(1:N, IG)) in / out.  cols: GP_NSTATE column pointers;
- * props: GP_NPROP column pointers.  Download returns the caller's original order. */
+ * props: GP_NPROP column pointers.  Download returns the caller's original order.  In
+ * gp_put_state, gp_download_state and gp_download_class with on_device, a column that ends
+ * before its n values is GP_EBADARG. */
 int gp_upload_state(gp_ctx *ctx, int64_t n, const double *const *cols,
                     const double *const *props, int32_t on_device);
 int gp_download_state(gp_ctx *ctx, int64_t n, double *const *cols, double *const *fluid,
